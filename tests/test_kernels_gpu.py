@@ -215,6 +215,24 @@ def test_attention_generic(dtype, nq, nkv, hd, P, window):
         assert torch.allclose(out[i].float().cpu().view(nq, hd), ref, **tol(dtype)), f"row {i} (request {r}, position {p})"
 
 
+@pytest.mark.parametrize("a_dtype,w_dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 256), (2, 41, 260), (3, 1000, 1024), (7, 24, 3080), (9, 8, 16), (64, 72, 520), (5, 9500, 264), (8, 16, 12288)])
+def test_gemm_generic_few_rows(a_dtype, w_dtype, M, N, K):
+    """The weight stream (up to 32 rows, narrow products up to 64): remainders of its 8 weight rows, of its runs of 1,024 terms and of its row groups, several
+    groups of weight rows in a block, K beyond one run of its warps. The sums are those of the tile kernel, bit for bit."""
+    from openinfer_b200.kernels import ops
+    a = torch.randn(M, K, device=DEV).to(a_dtype)
+    w = torch.randn(N, K, device=DEV).to(w_dtype)
+    out = torch.empty(M, N, device=DEV, dtype=torch.float32)
+    ops.gemm_generic(out, a, w)
+    ref = a.double() @ w.double().t()
+    # 256 sums of products of unit normals, then K / 256 partial sums: rounding 2^-24 of running totals of about sqrt(K)
+    assert (out.double() - ref).abs().max() < 2.0 ** -24 * (16 + (K / 256) ** 0.5) * 8 * K ** 0.5
+    many = torch.empty(65, N, device=DEV, dtype=torch.float32)
+    ops.gemm_generic(many, torch.cat([a, torch.zeros(65 - M, K, device=DEV, dtype=a_dtype)]), w)
+    assert torch.equal(many[:M], out)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_finds_one_far_key(dtype):
     """One key among hundreds is made to stand out (scaled query and key): the output must be
