@@ -233,6 +233,27 @@ def test_gemm_generic_few_rows(a_dtype, w_dtype, M, N, K):
     assert torch.equal(many[:M], out)
 
 
+@pytest.mark.parametrize("S", [1, 31, 32, 33, 255, 256, 257, 289, 1000])
+@pytest.mark.parametrize("window", [None, 40])
+def test_attention_generic_key_tiles(S, window):
+    """One float32 row over S keys: fewer and more key tiles than warps, remainders of a tile, a window."""
+    from openinfer_b200.kernels import ops
+    nq, nkv, hd, P = 4, 2, 128, 16
+    k, v, q = torch.randn(S, nkv, hd), torch.randn(S, nkv, hd), torch.randn(1, nq, hd)
+    pages = -(-S // P)
+    order = torch.randperm(pages).tolist()
+    cache = _paged(k, v, P, order, torch.float32, pages).to(DEV)
+    out = torch.empty(1, nq * hd, device=DEV)
+    ops.attention_generic(q.view(1, -1).to(DEV), out, cache[:, 0, 0], cache[:, 0, 1], cache.stride(0), P,
+                          torch.tensor([order], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV),
+                          torch.tensor([S - 1], dtype=torch.int32, device=DEV), nq, nkv, hd, hd ** -0.5, window)
+    lo = 0 if window is None else max(0, S - window)
+    for h in range(nq):
+        p = torch.softmax((k[lo:, h // 2].double() @ q[0, h].double()) * hd ** -0.5, dim=0)
+        # weights that add up to 1, values of a few units, some 10 roundings each
+        assert (out[0].view(nq, hd)[h].double().cpu() - p @ v[lo:, h // 2].double()).abs().max() < 5e-6
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_finds_one_far_key(dtype):
     """One key among hundreds is made to stand out (scaled query and key): the output must be
