@@ -120,6 +120,34 @@ __device__ __forceinline__ void store_accumulator(unsigned tmem_acc, TOut* __res
   }
 }
 
+// The same for a tile of grouped products (256 columns; with the activation 128 gate columns, then their 128 up columns, and
+// the activation in full precision as in the experts' other kernels). `dst`: the row's first element in C.
+template <typename TOut, bool kGlu>
+__device__ __forceinline__ void store_grouped(unsigned tmem_acc, TOut* __restrict__ dst, bool live, int n0, int N, int act, int part, float limit) {
+  constexpr int kCols = (kGlu ? 128 : 256) / kParts;
+#pragma unroll 1
+  for (int c = part * kCols; c < (part + 1) * kCols; c += 32) {
+    if (n0 + c >= N) break;                      // the same for the whole warp
+    unsigned v[32];
+    float a[32];
+    tmem_ld32(tmem_acc + (unsigned)c, v);
+    if constexpr (kGlu) {
+      unsigned u[32];
+      tmem_ld32(tmem_acc + 128u + (unsigned)c, u);
+      tmem_ld_wait();
+      if (live) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) a[e] = glu_act<false>(__uint_as_float(v[e]), __uint_as_float(u[e]), act, limit);
+      }
+    } else {
+      tmem_ld_wait();
+#pragma unroll
+      for (int e = 0; e < 32; ++e) a[e] = __uint_as_float(v[e]);
+    }
+    if (live) store_32(dst + n0 + c, a, N - (n0 + c));
+  }
+}
+
 // Persistent: CTA b works on tiles b, b + gridDim.x, ... (row tiles fastest, so CTAs that run at the
 // same time share W tiles through L2). The accumulator is double buffered in tensor memory
 // (2 x BN columns): while the epilogue warps drain tile i, the MMA warp already fills tile i + 1.
@@ -269,11 +297,30 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 //              "accumulator drained" barrier (16 arrivals).
 // Loads carry no cluster multicast: each CTA fetches what it holds. Every wait is bounded as above;
 // the two CTAs meet at the cluster's barrier before the tensor memory is freed.
-template <int kStages, typename TOut, bool kSiluMul>
+//
+// kGrouped: the products of routed experts (moe.cu). A's rows are (row, choice) pairs sorted by expert, W holds the
+// experts' matrices one below the other, and a row tile is an entry of a list that the device wrote: expert, first place,
+// up to 256 places. Every tile reads its expert's rows of W; places beyond the tile's are computed and not stored. With
+// the activation a tile's columns are 128 gate rows (the even CTA's half of W) and the 128 up rows of the same indices
+// (the odd CTA's), so W keeps its order of all gate rows, then all up rows. A tile of few places costs what its weights
+// cost to read, so the list's tiles need not be full: 16 experts of 2,048 x 1,536 with 770 places each take 149 us and 107 us
+// (the mma.sync tiles of 128 places: 653 us and 393 us).
+struct Groups {
+  const int* tiles;     // [3 * max_tiles]: expert, first place, places; then their number
+  const int* sorted;    // place -> pair
+  int max_tiles;
+  int expert_rows;      // rows of W per expert
+  int odd_offset;       // where the odd CTA's rows of W start, from the even CTA's
+  int scatter;          // results go to row sorted[place], else to row place
+};
+
+template <int kStages, typename TOut, bool kSiluMul, bool kGrouped = false>
 __global__ void __launch_bounds__(kThreads)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                         TOut* __restrict__ C, long long ldc, int M, int N, int K, int act, float act_p0, float act_p1) {
-  pdl_start();
+                         TOut* __restrict__ C, long long ldc, int M, int N, int K, int act, float act_p0, float act_p1,
+                         const Groups groups) {
+  if constexpr (kGrouped) pdl_wait();      // no early trigger: the next kernel's blocks would wait beside this product's
+  else pdl_start();
   constexpr int BN = 256, kPairM = 256;
   using L = Smem<128, kStages>;             // per CTA: 128 rows of A and 128 rows of W per stage
   extern __shared__ unsigned char smem_raw[];
@@ -290,7 +337,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int m_tiles = (M + kPairM - 1) / kPairM, n_tiles = (N + BN - 1) / BN;
+  constexpr int kStepN = kGrouped && kSiluMul ? BN / 2 : BN;      // N: output columns where tiles are grouped, else rows of W
+  const int m_tiles = kGrouped ? min(groups.tiles[3 * groups.max_tiles], groups.max_tiles) : (M + kPairM - 1) / kPairM;
+  const int n_tiles = (N + kStepN - 1) / kStepN;
   const int num_tiles = m_tiles * n_tiles;
   const int num_kb = (K + BK - 1) / BK;
 
@@ -322,7 +371,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       long long it = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const int m0 = (tile % m_tiles) * kPairM + (int)rank * 128, n0 = (tile / m_tiles) * BN + (int)rank * 128;
+        int m0 = (tile % m_tiles) * kPairM + (int)rank * 128, n0 = (tile / m_tiles) * kStepN + (int)rank * 128;
+        if constexpr (kGrouped) {
+          const int* t = groups.tiles + 3 * (tile % m_tiles);
+          m0 = t[1] + (int)rank * 128;
+          n0 = t[0] * groups.expert_rows + (tile / m_tiles) * kStepN + (int)rank * groups.odd_offset;
+        }
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = (int)(it % kStages);
           if (it >= kStages && !mbar_wait(empty_bar(s), (unsigned)((it / kStages) - 1) & 1, abort_flag, 1)) { ok = false; break; }
@@ -373,10 +427,17 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int a = local & 1;
       if (!mbar_wait(acc_full_bar(a), (unsigned)(local >> 1) & 1, abort_flag, 3)) break;
       tc_fence_after();
-      const int m0 = (tile % m_tiles) * kPairM + (int)rank * 128, n0 = (tile / m_tiles) * BN;
-      const int row = m0 + quarter * 32 + lane;
       const unsigned tmem_acc = tmem_base + (unsigned)(a * BN) + ((unsigned)(quarter * 32) << 16);
-      store_accumulator<BN, TOut, kSiluMul>(tmem_acc, C, ldc, row, n0, M, N, act, part, act_p0, act_p1);
+      if constexpr (kGrouped) {
+        const int* t = groups.tiles + 3 * (tile % m_tiles);
+        const int local_row = (int)rank * 128 + quarter * 32 + lane, place = t[1] + local_row;
+        const bool live = local_row < t[2];
+        const int row = live ? (groups.scatter ? groups.sorted[place] : place) : 0;
+        store_grouped<TOut, kSiluMul>(tmem_acc, C + (size_t)row * ldc, live, (tile / m_tiles) * kStepN, N, act, part, act_p0);
+      } else {
+        const int m0 = (tile % m_tiles) * kPairM + (int)rank * 128, n0 = (tile / m_tiles) * BN;
+        store_accumulator<BN, TOut, kSiluMul>(tmem_acc, C, ldc, m0 + quarter * 32 + lane, n0, M, N, act, part, act_p0, act_p1);
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_rank(acc_empty_bar(a), 0));
@@ -450,7 +511,30 @@ int launch_pair(void* C, long long ldc, const void* A, long long lda, const void
   }
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256);
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
-  oi_launch_cluster(kernel, 2 * pairs, kThreads, smem, s, 2, ma, mb, (TOut*)C, ldc, M, N, K, act, p0, p1);
+  oi_launch_cluster(kernel, 2 * pairs, kThreads, smem, s, 2, ma, mb, (TOut*)C, ldc, M, N, K, act, p0, p1, Groups{});
+  OI_CHECK_LAUNCH();
+  return OI_OK;
+}
+
+// every pair of SMs gets a pair of CTAs: how many tiles there are only the device knows
+template <typename TOut, bool kGlu>
+int launch_grouped(void* C, long long ldc, const void* A, long long rows, const void* W, int experts, int N, int K, int act, float limit,
+                   const int* tiles, int max_tiles, const int* sorted, int scatter, cudaStream_t s) {
+  const int expert_rows = kGlu ? 2 * N : N;
+  CUtensorMap ma, mb;
+  int rc = tc::make_map_2d_bf16(&ma, A, rows, K, K, 128);
+  OI_REQUIRE(rc == 0, "gemm_tcgen05_grouped: tensor map for A failed (%d; -1: cuTensorMapEncodeTiled is not available)", rc);
+  rc = tc::make_map_2d_bf16(&mb, W, (long long)experts * expert_rows, K, K, 128);
+  OI_REQUIRE(rc == 0, "gemm_tcgen05_grouped: tensor map for W failed (%d)", rc);
+  auto kernel = gemm_tcgen05_pair_kernel<kPairStages, TOut, kGlu, true>;
+  constexpr int smem = Smem<128, kPairStages>::kTotal;
+  static const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  OI_CHECK_CUDA(allowed);
+  int dev = 0, sms = 0;
+  OI_CHECK_CUDA(cudaGetDevice(&dev));
+  OI_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const Groups groups = {tiles, sorted, max_tiles, expert_rows, kGlu ? N : 128, scatter};
+  oi_launch_cluster(kernel, sms / 2 * 2, kThreads, smem, s, 2, ma, mb, (TOut*)C, ldc, (int)rows, N, K, act, limit, 0.f, groups);
   OI_CHECK_LAUNCH();
   return OI_OK;
 }
@@ -535,6 +619,20 @@ OI_API int oi_gemm_tcgen05_unary(void* C, int c_dtype, long long ldc, const void
     return pair ? launch_pair<kPairStages, float>(C, ldc, A, lda, W, ldw, M, N, K, s, act, p0, p1)
                 : launch<256, 4, float>(C, ldc, A, lda, W, ldw, M, N, K, s, act, p0, p1);
   OI_REQUIRE(false, "gemm_tcgen05_unary: unknown output dtype code %d", c_dtype);
+}
+
+// The grouped products of routed experts (256 x 256 tiles by pairs of CTAs): C[place or sorted[place], :] = A[place, :] W_e^T
+// for the places of every tile of the list `tiles` (see Groups). A [rows, K], dense. act == OI_ACT_NONE: W [experts, N, K],
+// C float32; otherwise W [experts, 2 N, K] (N gate rows, then N up rows) and C bfloat16 = the gated activation.
+OI_API int oi_gemm_tcgen05_grouped(void* C, long long ldc, const void* A, long long rows, const void* W, int experts, int N, int K,
+                                   int act, float limit, const int* tiles, int max_tiles, const int* sorted, int scatter, void* stream) {
+  OI_REQUIRE(rows >= 1 && experts >= 1 && N >= 1 && K >= 8 && K % 8 == 0, "gemm_tcgen05_grouped: bad sizes N=%d K=%d", N, K);
+  OI_REQUIRE((long long)experts * 2 * N < (1LL << 31), "gemm_tcgen05_grouped: %d experts of %d rows are too many", experts, N);
+  OI_REQUIRE((uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0, "gemm_tcgen05_grouped: operands must be 16-byte aligned");
+  cudaStream_t s = (cudaStream_t)stream;
+  if (act == OI_ACT_NONE)
+    return launch_grouped<float, false>(C, ldc, A, rows, W, experts, N, K, act, limit, tiles, max_tiles, sorted, scatter, s);
+  return launch_grouped<bf16, true>(C, ldc, A, rows, W, experts, N, K, act, limit, tiles, max_tiles, sorted, scatter, s);
 }
 
 // 0 when no bounded wait has run out since the last call; otherwise which role gave up

@@ -11,16 +11,20 @@
 //                          times the choice's weight is added in step 4)
 //   2. moe_group_kernel    the (row, choice) pairs sorted by expert (stable, so the order never depends on timing), and
 //                          the list of row tiles (expert, first sorted place, rows) the products run over
-//   3. moe_gemm_kernel     per tile: act(x W_gate_e^T, x W_up_e^T) for the rows of the tile, gathered by their pair's row;
+//   3. the products        per tile: act(x W_gate_e^T, x W_up_e^T) for the rows of the tile, gathered by their pair's row;
 //                          then the down projection, each row written to its pair's place
 //   4. moe_combine_kernel  out[row] = sum_j weight[row, j] * y[row * top + j], j ascending
 //
-// Steps of few rows (at most two pairs an expert on average) skip 2 and run 3 pair by pair (moe_gemv_kernel: a warp per
-// output row, the expert's rows read 16 bytes at a time); larger steps take the tiles.
+// Steps of few rows (at most two pairs an expert on average) skip 2 and stream every chosen expert's weights through the
+// tensor cores once (moe_stream.cu). Larger steps take tcgen05 tiles of 256 places (gemm_tcgen05.cu, over rows that
+// moe_gather_kernel has sorted): a tile of a few places costs what its expert's weights cost to read, so this holds from
+// the smallest such step on. Both want bfloat16 rows that TMA can read; other rows go pair by pair (moe_gemv_kernel: a
+// warp per output row) or by tiles of 32 places on the ordinary pipes. In batch-invariant mode the tiles of 32 and
+// 128 places on mma.sync take steps of any size, with the same sums.
 // Everything a step needs is found on the device (no sizes travel back to the host), so a step of single tokens can be
-// recorded and replayed. A row's sums are formed in the same order whatever else shares its tile: the result of a row does
-// not depend on the batch. The tiles' products run on the tensor cores for bfloat16 operands (mma.sync, float32
-// accumulation) and on the ordinary pipes for float32 and for rows that cannot be read 16 bytes at a time.
+// recorded and replayed. A row's sums are formed in the same order whatever else shares its tile.
+#include <type_traits>
+
 #include "oi_api.h"
 
 namespace {
@@ -28,63 +32,12 @@ namespace {
 constexpr int kTileM = 32, kTileN = 64, kTileK = 32;
 constexpr int kMaxTop = 32;
 
-template <typename T>
-__global__ void moe_router_kernel(const T* __restrict__ x, long long ldx, const void* __restrict__ w, int w_dtype, int rows, int K,
-                                  int E, int top, int* __restrict__ ids, float* __restrict__ wts, int scoring,
-                                  const float* __restrict__ correction, int n_groups, int keep_groups, float weight_scale) {
-  pdl_start();
-  extern __shared__ float smem[];              // the row's logits [E], scores [E], group scores [E], then which are taken [E bytes]
-  const int warps = blockDim.x >> 5, wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* z = smem;
-  float* sc = smem + E;
-  float* gs = smem + 2 * E;
-  unsigned char* taken = reinterpret_cast<unsigned char*>(smem + 3 * E);
-  const int row = blockIdx.x;
-  const T* xr = x + (size_t)row * ldx;
-  constexpr int kVec = 16 / (int)sizeof(T);
-  const bool vec = w_dtype == (sizeof(T) == 2 ? OI_BF16 : OI_F32) && K % kVec == 0 && ldx % kVec == 0 && (uintptr_t)x % 16 == 0 &&
-                   (uintptr_t)w % 16 == 0;
-  // one block a row; a warp takes four experts at a time, so that their loads are in flight together
-  for (int e0 = wi * 4; e0 < E; e0 += warps * 4) {
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    if (vec) {       // a lane takes 16 bytes of the row and of each expert's weights at a time
-      const T* wt = reinterpret_cast<const T*>(w);
-      // (experts beyond the last read the last one's row again and are not stored: loads without a condition can all be
-      // in flight at once, where a load behind a test waits for the one before it: 8 rows of width 2,048 21.8 -> 8.2 us)
-      const T* wrow[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) wrow[i] = wt + (size_t)min(e0 + i, E - 1) * K;
-#pragma unroll 2
-      for (int k = lane * kVec; k < K; k += 32 * kVec) {
-        T xv[kVec], wv[4][kVec];
-        *reinterpret_cast<uint4*>(xv) = *reinterpret_cast<const uint4*>(xr + k);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(wv[i]) = *reinterpret_cast<const uint4*>(wrow[i] + k);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int e = 0; e < kVec; ++e) acc[i] += to_f32(wv[i][e]) * to_f32(xv[e]);
-      }
-    } else {
-#pragma unroll 4
-      for (int k = lane; k < K; k += 32) {
-        const float xv = to_f32(xr[k]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (e0 + i < E) acc[i] += load_as_f32(w, w_dtype, (size_t)(e0 + i) * K + k) * xv;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float sum = warp_sum(acc[i]);
-      if (lane == 0 && e0 + i < E) {
-        z[e0 + i] = sum;
-        taken[e0 + i] = 0;
-      }
-    }
-  }
-  __syncthreads();
-  if (wi != 0) return;
+// One warp: the choice of one row from its logits z (behind them room for scores and group scores, [E] each).
+__device__ __forceinline__ void choose(float* z, unsigned char* taken, int row, int E, int top, int* __restrict__ ids, float* __restrict__ wts,
+                                       int scoring, const float* __restrict__ correction, int n_groups, int keep_groups, float weight_scale) {
+  const int lane = threadIdx.x & 31;
+  float* sc = z + E;
+  float* gs = z + 2 * E;
   if (scoring != 0) {
     float top_z = -INFINITY, sum = 0.f;
     if (scoring == 2) {                              // softmax over all of them
@@ -187,10 +140,79 @@ __global__ void moe_router_kernel(const T* __restrict__ x, long long ldx, const 
   }
 }
 
+// A block takes kRows rows, a warp kExperts experts at a time for all of them, and then chooses for row after row. Few rows:
+// 1 x 1, so that a row's 16-byte loads are all in flight (a warp per four experts took 14.5 us for 4 rows of width 2,048 and
+// 16 experts, this 7.3 us); many: 4 x 4, sixteen dot products for every eight loads (6,300 rows 39 us; one row a block took
+// 51 us, 4 x 1 69 us).
+template <typename T, int kRows, int kExperts>
+__global__ void __launch_bounds__(kRows > 1 ? 512 : 1024) moe_router_kernel(const T* __restrict__ x, long long ldx, const void* __restrict__ w, int w_dtype,
+                                                          int rows, int K, int E, int top, int* __restrict__ ids, float* __restrict__ wts,
+                                                          int scoring, const float* __restrict__ correction, int n_groups, int keep_groups,
+                                                          float weight_scale) {
+  pdl_start();
+  // per row: logits [E], scores [E], group scores [E]; then, per row, which experts are taken [E bytes]
+  extern __shared__ float smem[];
+  const int warps = blockDim.x >> 5, wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = blockIdx.x * kRows;
+  constexpr int kVec = 16 / (int)sizeof(T);
+  const bool vec = w_dtype == (sizeof(T) == 2 ? OI_BF16 : OI_F32) && K % kVec == 0 && ldx % kVec == 0 && (uintptr_t)x % 16 == 0 &&
+                   (uintptr_t)w % 16 == 0;
+  const T* xr[kRows];        // rows beyond the last read that one again and are not stored
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) xr[r] = x + (size_t)min(row0 + r, rows - 1) * ldx;
+  for (int e0 = wi * kExperts; e0 < E; e0 += warps * kExperts) {
+    float acc[kRows][kExperts] = {};
+    if (vec) {               // a lane takes 16 bytes of the rows and of the experts' weights at a time
+      const T* wrow[kExperts];      // experts beyond the last read that one again and are not stored
+#pragma unroll
+      for (int q = 0; q < kExperts; ++q) wrow[q] = reinterpret_cast<const T*>(w) + (size_t)min(e0 + q, E - 1) * K;
+#pragma unroll(kRows > 1 ? 1 : 8)
+      for (int k = lane * kVec; k < K; k += 32 * kVec) {
+        uint4 xv[kRows], wv[kExperts];
+#pragma unroll
+        for (int q = 0; q < kExperts; ++q) wv[q] = *reinterpret_cast<const uint4*>(wrow[q] + k);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) xv[r] = *reinterpret_cast<const uint4*>(xr[r] + k);
+#pragma unroll
+        for (int i = 0; i < kVec; ++i)
+#pragma unroll
+          for (int q = 0; q < kExperts; ++q)
+#pragma unroll
+            for (int r = 0; r < kRows; ++r)
+              acc[r][q] += to_f32(reinterpret_cast<const T*>(&wv[q])[i]) * to_f32(reinterpret_cast<const T*>(&xv[r])[i]);
+      }
+    } else {
+#pragma unroll 4
+      for (int k = lane; k < K; k += 32) {
+#pragma unroll
+        for (int q = 0; q < kExperts; ++q) {
+          const float wv = e0 + q < E ? load_as_f32(w, w_dtype, (size_t)(e0 + q) * K + k) : 0.f;
+#pragma unroll
+          for (int r = 0; r < kRows; ++r) acc[r][q] += wv * to_f32(xr[r][k]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int q = 0; q < kExperts; ++q) {
+        const float sum = warp_sum(acc[r][q]);
+        if (lane == 0 && e0 + q < E) {
+          smem[(size_t)r * 3 * E + e0 + q] = sum;
+          reinterpret_cast<unsigned char*>(smem + (size_t)kRows * 3 * E)[(size_t)r * E + e0 + q] = 0;
+        }
+      }
+  }
+  __syncthreads();
+  for (int r = wi; r < kRows && row0 + r < rows; r += warps)
+    choose(smem + (size_t)r * 3 * E, reinterpret_cast<unsigned char*>(smem + (size_t)kRows * 3 * E) + (size_t)r * E, row0 + r, E, top, ids, wts,
+           scoring, correction, n_groups, keep_groups, weight_scale);
+}
 // One block per expert e. sorted[first_e + i] = the i-th pair (in ascending pair number) that chose e; tiles of tile_m
 // sorted places that belong to one expert: tile_info[3 * t] = expert, first place, rows. tile_info's last word
 // (at 3 * max_tiles) is the number of tiles.
-__global__ void moe_group_kernel(const int* __restrict__ ids, int pairs, int E, int* __restrict__ sorted, int* __restrict__ tile_info,
+constexpr int kGroupThreads = 1024;      // (256 took 25 us for 12,600 pairs)
+__global__ void __launch_bounds__(kGroupThreads) moe_group_kernel(const int* __restrict__ ids, int pairs, int E, int* __restrict__ sorted, int* __restrict__ tile_info,
                                  int max_tiles, int tile_m) {
   pdl_start();
   extern __shared__ int hist[];       // [E] counts, then [warps] scan scratch
@@ -456,6 +478,7 @@ __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const bf16* __restric
 // of 32 k arrive by cp.async in two buffers, so that a tile's copies run beside the products of the one before. A row's
 // sums are formed in the same order as in the kernel above.
 constexpr int kBigM = 128;
+constexpr int kPairM = 256;     // places per tile of the tcgen05 products (gemm_tcgen05.cu)
 
 __device__ __forceinline__ void moe_cp16(void* dst, const void* src, bool valid) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -566,6 +589,21 @@ __global__ void __launch_bounds__(256) moe_gemm_mma_big_kernel(const bf16* __res
           out[row * ld_out + n] = from_f32<TO>(v);
         }
     }
+}
+
+// The rows of the pairs sorted by expert, 16 bytes a thread (a row has K / 8 pieces): the first product's tiles are then
+// plain boxes of rows.
+__global__ void moe_gather_kernel(bf16* __restrict__ dst, const bf16* __restrict__ x, long long ldx, int top, const int* __restrict__ sorted,
+                                  const int* __restrict__ tile_info, int max_tiles, int K) {
+  pdl_start();
+  const int tiles = min(tile_info[3 * max_tiles], max_tiles);
+  if (tiles == 0) return;
+  const int places = tile_info[3 * (tiles - 1) + 1] + tile_info[3 * (tiles - 1) + 2], pieces = K / 8;
+  const size_t n = (size_t)places * pieces;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int place = (int)(i / pieces), c = (int)(i - (size_t)place * pieces) * 8;
+    *reinterpret_cast<uint4*>(dst + (size_t)place * K + c) = *reinterpret_cast<const uint4*>(x + (size_t)(sorted[place] / top) * ldx + c);
+  }
 }
 
 // The same two products for steps of few rows (at most two pairs an expert on average): one block per (pair, 16 output
@@ -705,9 +743,13 @@ int launch_combine(float* out, const float* y, const float* wts, int top, int W,
 
 OI_API int oi_moe_max_tiles(int pairs, int experts) { return pairs / kTileM + experts; }
 
-// Sorted places per tile: 128 where the experts have 64 rows and more on average (the weights are then read once per 128
-// rows), otherwise 32 (fewer rows that are computed for nothing). A function of the step's size alone.
-OI_API int oi_moe_tile_rows(int pairs, int experts) { return (long long)pairs >= 64LL * experts ? kBigM : kTileM; }
+// Sorted places per tile: what a pair of CTAs of the tcgen05 product takes. In batch-invariant mode, whose sums are those of the
+// mma.sync tiles whatever the step's size, 128 where the experts have 64 rows and more on average (the weights are then
+// read once per 128 rows), otherwise 32 (fewer rows that are computed for nothing). A function of the step's size alone.
+OI_API int oi_moe_tile_rows(int pairs, int experts) {
+  if (!oi_option(OI_OPT_BATCH_INVARIANT)) return kPairM;
+  return (long long)pairs >= 64LL * experts ? kBigM : kTileM;
+}
 
 // Steps of at most this many (row, choice) pairs take the row-by-row products and need no grouping.
 // (None in batch-invariant mode, where a row's sums must be formed the same way whatever else is in the step.)
@@ -740,20 +782,27 @@ OI_API int oi_moe_route_scored(const void* x, int dtype, long long ldx, const vo
              "moe_route: %d experts in %d groups of which %d are kept cannot give %d choices", all, n_groups, keep_groups, top);
   if (rows == 0) return OI_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  const size_t smem = 3 * (size_t)all * sizeof(float) + (size_t)all + 16;
-  const int threads = all <= 16 ? 128 : (all >= 32 ? 256 : 32 * ((all + 3) / 4));      // a warp takes four experts at a time
-  if (dtype == OI_F32)
-    oi_launch(moe_router_kernel<float>, rows, threads, smem, s, (const float*)x, ldx, w_router, w_dtype, rows, K, all, top, ids, wts, scoring,
-              correction, n_groups, keep_groups, weight_scale);
-  else if (dtype == OI_BF16)
-    oi_launch(moe_router_kernel<bf16>, rows, threads, smem, s, (const bf16*)x, ldx, w_router, w_dtype, rows, K, all, top, ids, wts, scoring,
-              correction, n_groups, keep_groups, weight_scale);
-  else
+  // four rows a block where there are enough rows to give every SM several blocks all the same
+  constexpr int kMany = 4;
+  const bool many = rows >= 8 * 148 && all <= 512;
+  const int per_block = many ? kMany : 1, blocks = (rows + per_block - 1) / per_block;
+  const size_t smem = per_block * (3 * (size_t)all * sizeof(float) + (size_t)all) + 16;
+  const int groups_of = many ? (all + 3) / 4 : all, threads = 32 * (groups_of > (many ? 16 : 32) ? (many ? 16 : 32) : groups_of);
+#define OI_ROUTER(T, ROWS)                                                                                                          \
+  oi_launch(moe_router_kernel<T, ROWS, ROWS>, blocks, threads, smem, s, (const T*)x, ldx, w_router, w_dtype, rows, K, all, top, ids, wts, \
+            scoring, correction, n_groups, keep_groups, weight_scale)
+  if (dtype == OI_F32) {
+    if (many) OI_ROUTER(float, kMany); else OI_ROUTER(float, 1);
+  } else if (dtype == OI_BF16) {
+    if (many) OI_ROUTER(bf16, kMany); else OI_ROUTER(bf16, 1);
+  } else {
     OI_REQUIRE(false, "moe_route: unknown dtype code %d", dtype);
+  }
+#undef OI_ROUTER
   OI_CHECK_LAUNCH();
   const int pairs = rows * top;
   if (oi_moe_small(pairs, E)) return OI_OK;      // few rows: the products go pair by pair and need no grouping
-  oi_launch(moe_group_kernel, E, 256, (size_t)(E + 8) * sizeof(int), s, (const int*)ids, pairs, E, sorted, tile_info, oi_moe_max_tiles(pairs, E), oi_moe_tile_rows(pairs, E));
+  oi_launch(moe_group_kernel, E, kGroupThreads, (size_t)(E + kGroupThreads / 32) * sizeof(int), s, (const int*)ids, pairs, E, sorted, tile_info, oi_moe_max_tiles(pairs, E), oi_moe_tile_rows(pairs, E));
   OI_CHECK_LAUNCH();
   return OI_OK;
 }
@@ -786,7 +835,7 @@ OI_API int oi_moe_route_table(const int* token_ids, const int* table, int rows, 
   oi_launch(moe_table_kernel, (pairs + 127) / 128, 128, 0, s, token_ids, table, rows, vocab, E, top, 1.f / (float)top, ids, wts);
   OI_CHECK_LAUNCH();
   if (oi_moe_small(pairs, E)) return OI_OK;
-  oi_launch(moe_group_kernel, E, 256, (size_t)(E + 8) * sizeof(int), s, (const int*)ids, pairs, E, sorted, tile_info, oi_moe_max_tiles(pairs, E), oi_moe_tile_rows(pairs, E));
+  oi_launch(moe_group_kernel, E, kGroupThreads, (size_t)(E + kGroupThreads / 32) * sizeof(int), s, (const int*)ids, pairs, E, sorted, tile_info, oi_moe_max_tiles(pairs, E), oi_moe_tile_rows(pairs, E));
   OI_CHECK_LAUNCH();
   return OI_OK;
 }
@@ -801,6 +850,15 @@ OI_API int oi_moe_experts(const void* x, int dtype, long long ldx, const void* w
   if (rows == 0) return OI_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const int pairs = rows * top, max_tiles = oi_moe_max_tiles(pairs, E);
+  const bool tma = dtype == OI_BF16 && W % 8 == 0 && F % 8 == 0 && ldx % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)act % 16 == 0 &&
+                   (uintptr_t)w_gate_up % 16 == 0 && (uintptr_t)w_down % 16 == 0;
+  if (oi_moe_small(pairs, E) && tma && glu != OI_ACT_NONE) {
+    int rc = oi_moe_stream(act, F, x, ldx, rows, top, w_gate_up, E, F, W, glu, limit, ids, pairs, stream);
+    if (rc != OI_OK) return rc;
+    rc = oi_moe_stream(y, W, act, F, pairs, 1, w_down, E, W, F, OI_ACT_NONE, 0.f, ids, pairs, stream);
+    if (rc != OI_OK) return rc;
+    return launch_combine(out, y, wts, top, W, rows, add, ids, E, x, dtype, ldx, s);
+  }
   if (oi_moe_small(pairs, E) && (size_t)(W > F ? W : F) * sizeof(float) <= 48 * 1024) {
     const dim3 v1(pairs, (F + 15) / 16), v2(pairs, (W + 15) / 16);
     if (dtype == OI_F32) {
@@ -835,6 +893,18 @@ OI_API int oi_moe_experts(const void* x, int dtype, long long ldx, const void* w
     // tensor cores when every row of the operands starts on a 16-byte boundary
     const bool tc1 = W % 8 == 0 && ldx % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w_gate_up % 16 == 0;
     const bool tc2 = F % 8 == 0 && (uintptr_t)act % 16 == 0 && (uintptr_t)w_down % 16 == 0;
+    if (tma && tile_rows == kPairM && (uintptr_t)y % 16 == 0 && glu != OI_ACT_NONE) {
+      // the sorted rows lie where y will be: the second product writes it, the first reads it
+      const size_t pieces = (size_t)pairs * (W / 8);
+      const int blocks = (int)((pieces + 255) / 256 > 148 * 8 ? 148 * 8 : (pieces + 255) / 256);
+      oi_launch(moe_gather_kernel, blocks, 256, 0, s, (bf16*)y, (const bf16*)x, ldx, top, sorted, tile_info, max_tiles, W);
+      OI_CHECK_LAUNCH();
+      int rc = oi_gemm_tcgen05_grouped(act, F, y, pairs, w_gate_up, E, F, W, glu, limit, tile_info, max_tiles, sorted, 0, stream);
+      if (rc != OI_OK) return rc;
+      rc = oi_gemm_tcgen05_grouped(y, W, act, pairs, w_down, E, W, F, OI_ACT_NONE, 0.f, tile_info, max_tiles, sorted, 1, stream);
+      if (rc != OI_OK) return rc;
+      return launch_combine(out, y, wts, top, W, rows, add, ids, E, x, dtype, ldx, s);
+    }
     if (tc1 && big)
       oi_launch(moe_gemm_mma_big_kernel<bf16, true>, b1, 256, 0, s, (const bf16*)x, ldx, top, (const bf16*)w_gate_up, (long long)2 * F * W,
                 (bf16*)act, (long long)F, 0, sorted, tile_info, max_tiles, F, W, limit, glu);

@@ -192,9 +192,8 @@ def test_sum_of_sublayers_token_gate_and_table_routing_kernels():
                                                    (700, 72, 40, 3, 2, 16), (150, 64, 200, 2, 1, 0), (1100, 256, 136, 5, 3, 0)])
 def test_experts_by_table_kernels(dtype, rows, W, F, E, top, shared):
     """Experts chosen by the token id through a table, each weighted 1 / top, plus an expert every row uses, against the
-    plain statement row by row; a row's result does not depend on the rows beside it (steps whose experts have 64 rows and
-    more on average take tiles of 128 rows, smaller ones tiles of 32, the smallest go pair by pair: the last three cases
-    compare a row across them)."""
+    plain statement row by row; a row's result does not depend on the rows beside it (the last three cases compare a row
+    across steps that take tiles and steps that stream the chosen experts' weights, in float32 pair by pair)."""
     from openinfer_b200.kernels import ops
     g = torch.Generator().manual_seed(rows + E)
     vocab = 61

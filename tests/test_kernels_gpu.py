@@ -1198,3 +1198,54 @@ def test_attention_mma_long_contexts(nq, nkv, hd):
     each, block-table rounds of the TMA producer), and decode rows at 5,000 and 3,001 keys (32 key slices)."""
     plan = _mma_case(nq, nkv, hd, 16, None, [1500, 1, 1, 300], [3000, 5000, 3001, 300], seed=3)
     assert plan.num_tile_items and plan.num_decode_items
+
+
+# ------------------------------------------------------------------------------------------------ routed experts
+def _experts_reference(x, gate_up, down, ids, wts):
+    """Routed experts in float64 from the stored numbers, and a bound on what rounding the activations to bfloat16 (8 bits, so
+    2^-8 of each at most, all of one sign at worst) and the float32 sums may add."""
+    out, bound = [], []
+    for t in range(x.shape[0]):
+        o, b = 0.0, 0.0
+        for e, w in zip(ids[t].tolist(), wts[t].tolist()):
+            g, u = (gate_up[e].double() @ x[t].double()).chunk(2)
+            a = g * torch.sigmoid(g) * u
+            o = o + w * (down[e].double() @ a)
+            b = b + w * (down[e].double().abs() @ (a.abs() * 2.0 ** -8 + 1e-5))
+        out.append(o)
+        bound.append(b)
+    return torch.stack(out), torch.stack(bound)
+
+
+@pytest.mark.parametrize("rows,W,F,E,top", [
+    (3, 64, 48, 100, 2), (20, 256, 40, 70, 3), (16, 128, 96, 16, 2), (13, 264, 72, 33, 1), (1, 8, 136, 4, 1), (9, 2048, 1536, 16, 2),  # few rows
+    (40, 200, 72, 3, 2), (300, 264, 136, 5, 2), (600, 512, 384, 2, 1), (35, 64, 8, 40, 2), (1300, 72, 264, 4, 3)])   # tiles of 256 places
+@pytest.mark.parametrize("shape", ["spread", "one"])
+def test_routed_experts_bf16_sizes(rows, W, F, E, top, shape):
+    """Edges of the tcgen05 tiles (places, columns, columns of the last 64 along K) and of the weight stream of few rows (16, 32 and 64
+    rows of the second product, K slices), experts that nobody or that everybody chose, more experts than pairs."""
+    from openinfer_b200.kernels import gemm_tcgen05, ops
+    g = torch.Generator().manual_seed(rows + W)
+    x = torch.randn(rows, W, generator=g).to(torch.bfloat16).to(DEV)
+    gate_up = (torch.randn(E, 2 * F, W, generator=g) * W ** -0.5).to(torch.bfloat16).to(DEV)
+    down = (torch.randn(E, W, F, generator=g) * F ** -0.5).to(torch.bfloat16).to(DEV)
+    table = torch.stack([torch.randperm(E, generator=g)[:top] if shape == "spread" else torch.arange(E - top, E) for _ in range(rows)])
+    routing = ops.moe_route_table(torch.arange(rows, dtype=torch.int32, device=DEV), table.to(torch.int32).to(DEV), E)
+    out = ops.moe_experts(x, gate_up, down, routing, 0.0, act="silu").double()
+    ref, bound = _experts_reference(x, gate_up, down, routing[0], routing[1])
+    assert ((out - ref).abs() <= bound).all()
+    assert ops.moe_stream_status() == 0 and gemm_tcgen05.status() == 0
+
+
+@pytest.mark.parametrize("E,scoring,groups,keep", [(16, "softmax_top", 1, 1), (20, "sigmoid_groups", 4, 2), (40, "softmax_groups", 5, 3)])
+@pytest.mark.parametrize("K", [136, 2048])
+def test_router_rows_of_a_large_step(E, scoring, groups, keep, K):
+    """Steps of many rows take four rows a block: the same choices and weights, bit for bit, as rows that come a few at a time."""
+    from openinfer_b200.kernels import ops
+    x = torch.randn(1187, K, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(E, K, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    kw = {} if scoring == "softmax_top" else dict(scoring=scoring, correction=torch.randn(E, device=DEV) * 0.1, groups=groups, keep_groups=keep)
+    ids, wts, _, _ = ops.moe_route(x, w, 2, **kw)
+    for lo in (0, 600, 1180):
+        few_ids, few_wts, _, _ = ops.moe_route(x[lo: lo + 7].contiguous(), w, 2, **kw)
+        assert torch.equal(ids[lo: lo + 7], few_ids) and torch.equal(wts[lo: lo + 7], few_wts)
