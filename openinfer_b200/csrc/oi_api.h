@@ -324,8 +324,8 @@ OI_API int oi_argmax(int* out, const float* logits, int rows, int vocab, long lo
        int* partial_idx, void* stream);
 OI_API int oi_sample_use_clusters(int on);
 OI_API int oi_sample(int* out, const float* logits, long long row_stride, float* probs, int rows, int vocab, const
-       float* temperature, const int* top_k, const float* top_p, const float* min_p, const float* uniform, void*
-       stream);
+       float* temperature, const int* top_k, const float* top_p, const float* min_p, const float* uniform, const int*
+       row_idx, void* stream);
 OI_API int oi_token_logprobs(const float* logits, long long row_stride, int vocab, const int* rows, const int* picked,
        const int* ks, int n, int k_max, float* out_lp, float* top_vals, int* top_ids, void* stream);
 

@@ -325,26 +325,30 @@ def sample_use_clusters(on: bool) -> None:
 
 
 def sample(out: torch.Tensor, logits: torch.Tensor, probs_scratch: torch.Tensor, temperature: torch.Tensor,
-           top_k: torch.Tensor, top_p: torch.Tensor, min_p: torch.Tensor, uniform: torch.Tensor) -> torch.Tensor:
+           top_k: torch.Tensor, top_p: torch.Tensor, min_p: torch.Tensor, uniform: torch.Tensor,
+           row_idx: Optional[torch.Tensor] = None) -> torch.Tensor:
     """One token per row from softmax(logits / temperature) after top-k, top-p and min-p,
-    by inverse CDF at ``uniform[r]`` in [0, 1)."""
-    _cuda(out, logits, probs_scratch, temperature, top_k, top_p, min_p, uniform)
+    by inverse CDF at ``uniform[r]`` in [0, 1). With ``row_idx`` (int32, on the device) the parameters are those of the
+    rows it lists: their logits are read and their places of ``out`` written, the other places stay as they are."""
+    _cuda(out, logits, probs_scratch, temperature, top_k, top_p, min_p, uniform, row_idx)
     _i32(out, "sample out")
     _i32(top_k, "top_k")
-    rows, vocab = logits.shape
+    _i32(row_idx, "sample row_idx")
+    all_rows, vocab = logits.shape
+    rows = all_rows if row_idx is None else row_idx.numel()
     if logits.dtype != torch.float32 or logits.stride(1) != 1:
         raise KernelError("sample: logits must be float32 rows")
     for t, name in ((temperature, "temperature"), (top_p, "top_p"), (min_p, "min_p"), (uniform, "uniform")):
         if t.dtype != torch.float32 or t.numel() != rows or not t.is_contiguous():
             raise KernelError(f"sample: {name} must be float32 with one entry per row")
-    if top_k.numel() != rows or out.numel() != rows:
+    if top_k.numel() != rows or out.numel() != all_rows:
         raise KernelError("sample: top_k/out must have one entry per row")
     if probs_scratch.dtype != torch.float32 or probs_scratch.numel() < rows * vocab or not probs_scratch.is_contiguous():
         raise KernelError("sample: scratch must hold rows * vocab float32 values")
     L = _lib.load()
     _lib.check(L.oi_sample(out.data_ptr(), logits.data_ptr(), logits.stride(0), probs_scratch.data_ptr(), rows, vocab,
                            temperature.data_ptr(), top_k.data_ptr(), top_p.data_ptr(), min_p.data_ptr(),
-                           uniform.data_ptr(), _stream()), "sample")
+                           uniform.data_ptr(), _ptr(row_idx), _stream()), "sample")
     return out
 
 

@@ -98,15 +98,12 @@ class Sampler:
             fl = dev[: 4 * k].view(torch.float32).view(4, k)
             tk = dev[4 * k: 5 * k]
             idx = dev[5 * k: 6 * k]
-            rows = logits if k == n else logits.index_select(0, idx)
             if self._probs is None or self._probs.numel() < k * self.vocab_size:
                 self._probs = torch.empty(k * self.vocab_size, dtype=torch.float32, device=self.device)
-            picked = torch.empty(k, dtype=torch.int32, device=self.device)
-            ops.sample(picked, rows.contiguous(), self._probs, fl[0], tk, fl[1], fl[2], fl[3])
-            if k == n:
-                out = picked
-            else:
-                out.index_copy_(0, idx.to(torch.int64), picked)   # greedy rows keep their argmax
+            if logits.stride(1) != 1:
+                logits = logits.contiguous()
+            # the kernel reads the sampled rows where they are and writes their places: greedy rows keep their argmax
+            ops.sample(out, logits, self._probs, fl[0], tk, fl[1], fl[2], fl[3], row_idx=None if k == n else idx)
         host = self._host_buffer(n)
         ops.copy_words(host, out, n)     # a kernel writes the ids into pinned host memory: no copy-engine operation
         event = torch.cuda.Event()

@@ -368,6 +368,33 @@ def test_sample_matches_plain_distribution(vocab, sample_clusters):
             assert lo - 1e-4 <= u <= float(cdf[tok]) + 1e-4, f"setting {settings[r]} u={u}: token {tok} covers [{lo}, {float(cdf[tok])}]"
 
 
+@pytest.mark.parametrize("spread", [0.35, 1.0, 3.0])
+@pytest.mark.parametrize("vocab", [32768, 151936])
+def test_sample_by_clusters_keeps_what_one_block_keeps(vocab, spread):
+    """The thresholds that the clusters take from their sorted list (short, up to 2,048 and up to 4,096 values, with ties) are those of the
+    one-block kernel's radix selection: every uniform number draws the same token, for all rows and for listed ones. (Of a few
+    thousand values at most: among tens of thousands of equal ones the two kernels' float32 sums may part at a boundary.)"""
+    from openinfer_b200.kernels import ops
+    torch.manual_seed(vocab)
+    rows = 24
+    logits = (torch.randn(rows, vocab, device=DEV) * spread).mul(64).round().div(64)      # on a grid: many exact ties
+    i32 = dict(dtype=torch.int32, device=DEV)
+    T, K = torch.linspace(0.5, 1.2, rows, device=DEV), torch.tensor([(1, 2, 50, 300, 1023, 2049)[r % 6] for r in range(rows)], **i32)
+    P, MP = torch.tensor([(0.95, 1.0, 0.5, 0.02)[r % 4] for r in range(rows)], device=DEV), torch.zeros(rows, device=DEV)
+    scratch = torch.empty(rows * vocab, device=DEV)
+    for u in (0.0, 0.31, 0.62, 0.93):
+        U, got = torch.full((rows,), u, device=DEV), {}
+        for clusters in (True, False):
+            ops.sample_use_clusters(clusters)
+            got[clusters] = ops.sample(torch.empty(rows, **i32), logits, scratch, T, K, P, MP, U).tolist()
+        ops.sample_use_clusters(True)
+        assert got[True] == got[False]
+        idx = torch.tensor([21, 3, 8], **i32)
+        pick = lambda t: t[idx.long()].contiguous()      # noqa: E731
+        out = ops.sample(torch.full((rows,), 77, **i32), logits, scratch, pick(T), pick(K), pick(P), pick(MP), pick(U), row_idx=idx).tolist()
+        assert out == [got[True][r] if r in (21, 3, 8) else 77 for r in range(rows)]
+
+
 def test_sample_when_the_estimate_of_the_candidate_list_is_wrong(sample_clusters):
     """The kernel places the cut of its shared-memory list from a histogram of one value in eight (the first of
     every other group of four per thread). 5,000 equal large values at places that are never counted make that
