@@ -1219,6 +1219,28 @@ def test_token_logprobs(vocab):
         assert (ids[i, k:] == -1).all() and bool(torch.isinf(vals[i, k:]).all())
 
 
+@pytest.mark.parametrize("vocab", [1, 3, 2049, 32770])
+def test_token_logprobs_of_one_thread_and_odd_rows(vocab):
+    """Entries of one thread in a row (its next ones come from a second look), rows that do not start on 16 bytes, entries of minus
+    infinity, fewer entries than asked for."""
+    from openinfer_b200.kernels import ops
+    torch.manual_seed(vocab)
+    logits = torch.randn(3, vocab) * 2
+    for j, i in enumerate(range(5, vocab, 2048)):
+        logits[1, i] = 9.0 - 0.25 * (j // 2)               # pieces of thread 1, in ties of two
+    logits[2, 1:] = -float("inf")
+    i32 = dict(dtype=torch.int32, device=DEV)
+    lp, vals, ids = ops.token_logprobs(logits.to(DEV), torch.arange(3, **i32), torch.tensor([0, vocab - 1, 0], **i32), torch.tensor([7, 7, 7], **i32), 7)
+    ref = torch.log_softmax(logits.double(), dim=-1)
+    for r in range(3):
+        order = sorted(range(vocab), key=lambda j: (-float(logits[r, j]), j))[:7]
+        assert ids[r].tolist() == order + [-1] * (7 - len(order))
+        # one float32 rounding of the logarithm (2^-24 of some 10), one of the difference
+        want = ref[r, order]
+        assert torch.allclose(vals[r, : len(order)].cpu().double(), want, atol=4e-6)
+    assert torch.allclose(lp.cpu().double(), torch.stack([ref[0, 0], ref[1, vocab - 1], ref[2, 0]]), atol=4e-6)
+
+
 @pytest.mark.parametrize("nq,nkv,hd", [(4, 2, 128), (4, 1, 64)])
 def test_attention_mma_long_contexts(nq, nkv, hd):
     """Thousands of keys: a 1,500-token portion over a 1,500-token prefix (many query tiles, up to 47 key tiles
