@@ -122,15 +122,16 @@ class RunnerExecutor(Executor):
         tokens = dict(zip(ids, pending.result())) if pending is not None else {}
         if lp is not None:
             tok_ids, spans, ks, lpv, vals, tids = lp
-            lpv, vals, tids = lpv.cpu().tolist(), vals.cpu().tolist(), tids.cpu().tolist()
-
-            def entry(i):
-                return TokenLogprob(lpv[i], [(tids[i][j], vals[i][j]) for j in range(ks[i]) if tids[i][j] >= 0])
+            # a prompt scored with `echo` brings an entry per position: whole rows at a time, not number by number
+            tids = tids.cpu()
+            counts = torch.minimum((tids >= 0).sum(dim=1), torch.tensor(ks)).tolist()    # unused places hold -1, behind the used ones
+            tops = [list(zip(t[:n], v[:n])) for t, v, n in zip(tids.tolist(), vals.cpu().tolist(), counts)]
+            entries = list(map(TokenLogprob, lpv.cpu().tolist(), tops))
 
             for i, rid in enumerate(tok_ids):
-                self.last_logprobs.setdefault(rid, {})["token"] = entry(i)
+                self.last_logprobs.setdefault(rid, {})["token"] = entries[i]
             for rid, first_pos, at, n in spans:
-                got = [entry(at + j) for j in range(n)]
+                got = entries[at: at + n]
                 # position 0 of the prompt has nothing in front of it
                 self.last_logprobs.setdefault(rid, {})["prompt"] = ([None] if first_pos == 0 else []) + got
         return tokens
