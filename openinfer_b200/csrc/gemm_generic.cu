@@ -65,7 +65,6 @@ __global__ void gemm_rows_kernel(TC* __restrict__ C, const TA* __restrict__ A, c
                                  long long lda, long long ldw, long long ldc, int chunk_warps, int row_warps, int row_groups) {
   using L = Rows<TA, TW, MG>;
   constexpr int KS = L::KS, VW = 16 / (int)sizeof(TW), VA = 16 / (int)sizeof(TA), V = VW > VA ? VW : VA;
-  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cw = warp % chunk_warps, rw = warp / chunk_warps;
@@ -78,7 +77,7 @@ __global__ void gemm_rows_kernel(TC* __restrict__ C, const TA* __restrict__ A, c
   const int row = lane & 7, part = lane >> 3;
 
   for (int c0 = cw * 4; c0 < chunks; c0 += chunk_warps * 4) {
-    auto fetch = [&](int sub) {                    // the stage of terms [sub * KS, + KS) of the warp's four partial sums
+    auto fetch_w = [&](int sub) {                  // the stage of terms [sub * KS, + KS) of the warp's four partial sums
       const unsigned base = ring_addr + (unsigned)(sub % L::kStages) * L::kStage;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {                // 32 segments x 8 pieces of 16 bytes: 8 lanes fetch one segment
@@ -87,6 +86,9 @@ __global__ void gemm_rows_kernel(TC* __restrict__ C, const TA* __restrict__ A, c
         const int left = (n < N && k < K) ? (K - k < VW ? K - k : VW) : 0;
         cp_async_16(base + seg * L::kWSlot + piece * 16, left ? W + (size_t)n * ldw + k : W, left * (int)sizeof(TW));
       }
+    };
+    auto fetch_a = [&](int sub) {
+      const unsigned base = ring_addr + (unsigned)(sub % L::kStages) * L::kStage;
       constexpr int kPieces = L::kASeg / 16;
       for (int i = lane; i < 4 * MG * kPieces; i += 32) {
         const int seg = i / kPieces, piece = i % kPieces;
@@ -100,12 +102,16 @@ __global__ void gemm_rows_kernel(TC* __restrict__ C, const TA* __restrict__ A, c
 #pragma unroll
     for (int m = 0; m < MG; ++m) sum[m] = 0.f;
     __syncwarp();
+    // the weights' first stages before the wait for the kernel that forms A (no kernel of a step writes weights): kSub >= 4
 #pragma unroll
-    for (int s = 0; s < L::kStages - 1; ++s) fetch(s);             // kSub >= 4 stages
+    for (int s = 0; s < L::kStages - 1; ++s) fetch_w(s);
+    if (c0 == cw * 4) pdl_wait();
+#pragma unroll
+    for (int s = 0; s < L::kStages - 1; ++s) fetch_a(s);
     for (int sub = 0; sub < L::kSub; ++sub) {
       asm volatile("cp.async.wait_group %0;\n" ::"n"(L::kStages - 2) : "memory");
       __syncwarp();                                                // everybody's pieces are there, and the stage before is read
-      if (sub + L::kStages - 1 < L::kSub) fetch(sub + L::kStages - 1);
+      if (sub + L::kStages - 1 < L::kSub) fetch_w(sub + L::kStages - 1), fetch_a(sub + L::kStages - 1);
       else asm volatile("cp.async.commit_group;\n" ::: "memory");
       const unsigned char* st = ring + (size_t)(sub % L::kStages) * L::kStage;
       const TW* w = reinterpret_cast<const TW*>(st + lane * L::kWSlot);
