@@ -1298,3 +1298,72 @@ def test_router_rows_of_a_large_step(E, scoring, groups, keep, K):
     for lo in (0, 600, 1180):
         few_ids, few_wts, _, _ = ops.moe_route(x[lo: lo + 7].contiguous(), w, 2, **kw)
         assert torch.equal(ids[lo: lo + 7], few_ids) and torch.equal(wts[lo: lo + 7], few_wts)
+
+
+# ------------------------------------------------------------------------------------------------ recurrences
+@pytest.mark.parametrize("mode", ["matrix_memory", "gated_delta", "linear_decay"])
+@pytest.mark.parametrize("D,V", [(5, 7), (32, 33), (33, 8), (64, 100), (100, 64), (128, 130), (132, 9), (256, 32), (300, 17)])
+def test_recurrent_scan_runs_of_rows(mode, D, V):
+    """Rows are walked four at a time: requests of one to thirteen rows and of a few chunks, over old state, key channels around
+    every split over lanes, columns that do not fill a block, two heads per key head; row by row in float64."""
+    from types import SimpleNamespace
+
+    from openinfer_b200.kernels import ops
+    torch.manual_seed(D + V)
+    lens, H, G = [1, 2, 3, 4, 5, 9, 13, 42], 2, 1
+    T, B = sum(lens), len(lens)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    cu = [sum(lens[:b]) for b in range(B + 1)]
+    ctx = SimpleNamespace(cu_seqlens=torch.tensor(cu, **i32), token_req=torch.tensor([b for b, n in enumerate(lens) for _ in range(n)], **i32),
+                          state_slots=torch.tensor([(b * 3) % B for b in range(B)], **i32), state_phase=torch.tensor([b % 2 for b in range(B)], **i32),
+                          num_requests=B)
+    qkv = torch.randn(T, 2 * G * D + H * V, device=DEV)
+    gates = torch.randn(T, 2 * H, device=DEV)
+    delta, memory = mode == "gated_delta", mode == "matrix_memory"
+    state = torch.randn(B, 2, H, D * V + (D + 1 if memory else 0), device=DEV) * 0.3
+    if memory:
+        state[..., -1].abs_()
+    before = state.double().cpu()
+    decay = torch.randn(T, H * D, device=DEV)
+    p0 = torch.randn(H * D if delta else H, device=DEV) * 0.3
+    if not (delta or memory):
+        p0 = p0.sigmoid()
+    p1 = torch.randn(H, device=DEV) * 0.3
+    out = torch.empty(T, H * V, device=DEV)
+    code = ops.SCAN_GATED_DELTA if delta else ops.SCAN_MATRIX_MEMORY if memory else ops.SCAN_LINEAR_DECAY
+    x = qkv.double().cpu()          # (the linear decay turns the values into their silu in place)
+    ops.recurrent_scan(code, out, qkv, (0, G * D, 2 * G * D), gates, (0, H), state, ctx, H, G, D, V,
+                       p0=p0, p1=p1, decay=decay if delta else None, cap=15.0, q_scale=D ** -0.5)
+    g, dc, p0, p1 = (t.double().cpu() for t in (gates, decay, p0, p1))
+    if not (delta or memory):
+        x = torch.nn.functional.silu(x)
+    q, k, v = x[:, : G * D].view(T, G, D), x[:, G * D: 2 * G * D].view(T, G, D), x[:, 2 * G * D:].view(T, H, V)
+    for b in range(B):
+        slot, phase = (b * 3) % B, b % 2
+        for h in range(H):
+            old = before[slot, phase, h]
+            C, n, m = old[: D * V].view(V, D).clone(), old[D * V: D * V + D].clone(), old[-1].clone()
+            for t in range(cu[b], cu[b + 1]):
+                kt, qt, vt = k[t, 0], q[t, 0], v[t, h]
+                if delta:
+                    kt, qt = kt / (kt @ kt + 1e-6).sqrt(), qt / (qt @ qt + 1e-6).sqrt() * D ** -0.5
+                    C = C * torch.exp(-torch.exp(p1[h]) * torch.nn.functional.softplus(dc[t].view(H, D)[h] + p0.view(H, D)[h]))
+                    C = C + torch.outer(torch.sigmoid(g[t, h]) * (vt - C @ kt), kt)
+                    o = C @ qt
+                elif not memory:
+                    C = p0[h] * C + torch.outer(vt, kt)
+                    o = C @ (qt * D ** -0.5)
+                else:
+                    qt = qt * D ** -0.5
+                    i, f = 15 * torch.tanh((g[t, h] + p0[h]) / 15), torch.nn.functional.logsigmoid(15 * torch.tanh((g[t, H + h] + p1[h]) / 15))
+                    new = torch.maximum(f + m, i)
+                    C, n = torch.exp(f + m - new) * C + torch.exp(i - new) * torch.outer(vt, kt), torch.exp(f + m - new) * n + torch.exp(i - new) * kt
+                    m = new
+                    o = C @ qt / (torch.maximum((n @ qt).abs(), torch.exp(-m)) + 1e-6)
+                # 42 steps of sums of up to 300 float32 products: a few hundred roundings of 2^-24, and a denominator that may be small
+                bound = 3e-5 * (1 + C.abs().max() + o.abs().max() * (1 if not memory else 1 / (n @ qt).abs().clamp(min=float(torch.exp(-m)))))
+                assert (out[t].double().cpu().view(H, V)[h] - o).abs().max() < bound
+            got = state[slot, 1 - phase, h].double().cpu()
+            assert (got[: D * V].view(V, D) - C).abs().max() < 3e-5 * (1 + C.abs().max())
+            if memory:
+                assert (got[D * V: D * V + D] - n).abs().max() < 3e-5 * (1 + n.abs().max()) and abs(got[-1] - m) < 3e-5 * (1 + abs(m))
