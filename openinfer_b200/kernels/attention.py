@@ -137,6 +137,7 @@ DECODE_LONG_CONTEXT = 12288
 DECODE_VERY_LONG_CONTEXT = 24576   # and from here up to 128: batch 1 at 32,768 keys 240 against 229, at 65,536 206 against 188
 DECODE_VERY_LONG_SPLITS = 128
 DECODE_MIN_KEYS_PER_SPLIT = 32
+DECODE_KEYS_PER_RECORDED_SPLIT = 64   # of a recorded step's capacity: its rows hold half of that and more
 DECODE_MAX_GROUP = 16
 _SM_COUNT = None
 
@@ -209,6 +210,12 @@ def decode_splits(num_rows: int, nkv: int, sm_count: int, max_kv_len: Optional[i
         max_kv_len = min(chunk, max_kv_len) if max_kv_len is not None else chunk
     if max_kv_len is not None:
         ns = min(ns, max(DECODE_WARPS, (max_kv_len // DECODE_MIN_KEYS_PER_SPLIT) // DECODE_WARPS * DECODE_WARPS))
+    elif capacity is not None and ns <= DECODE_MAX_SPLITS:
+        # Slices that a short row cannot fill still take part in the merge and in the cluster's barrier. Passes of 32 decoded
+        # tokens, ms with 4 / 8 / 16 / 32 slices: Qwen3-0.6B sizes, batch 1, 60 keys 25.1 / 26.7 / 26.6 / 28.3, 200 keys 26.7 / 27.0 /
+        # 27.4 / 28.5, 400 keys 30.2 / 28.2 / 28.3 / 29.3, 900 keys 37.0 / 32.4 / 30.1 / 31.1; batch 4, 200 keys 30.5 / 30.4 / 31.0 /
+        # 33.4; Qwen3-8B sizes (16 layers), batch 1, 200 keys 50.8 / 50.1 / 50.0 / 50.3, 900 keys 58.4 / 55.0 / 53.5 / 53.7
+        ns = min(ns, max(DECODE_WARPS, capacity // DECODE_KEYS_PER_RECORDED_SPLIT // DECODE_WARPS * DECODE_WARPS))
     return ns
 
 
