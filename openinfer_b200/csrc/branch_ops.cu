@@ -159,12 +159,13 @@ __global__ void short_conv_kernel(TO* __restrict__ out, const TX* __restrict__ x
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void latent_store_kernel(T* __restrict__ pages, long long page_stride, int page_size, int row_elems,
-                                    const T* __restrict__ src, long long src_stride, const void* __restrict__ w, int w_dtype,
+                                    const T* src, long long src_stride, const void* __restrict__ w, int w_dtype,
                                     const int* __restrict__ slots, int rank, float eps, float w_offset) {
-  pdl_start();
+  pdl_trigger();
   __shared__ float red[32];
   const int t = blockIdx.x;
-  const int slot = slots[t];
+  const int slot = slots[t];      // (the step's metadata: before the wait)
+  pdl_wait();
   if (slot < 0) return;     // whole block leaves
   const T* z = src + (size_t)t * src_stride;
   float ss = 0.f;
@@ -236,8 +237,8 @@ __device__ __forceinline__ void store4(bf16* p, const float v[4]) {
 constexpr int kMaxCoef = 256;   // terms of an average the vector kernel keeps in shared memory
 
 template <typename TA, int VPT>
-__global__ void branch_norm_add_vec_kernel(float* __restrict__ h, const TA* __restrict__ a, const void* __restrict__ w, int w_dtype,
-                                           int hidden, float eps, float w_offset, float* __restrict__ hist, long long hist_stride,
+__global__ void branch_norm_add_vec_kernel(float* h, const TA* a, const void* __restrict__ w, int w_dtype,
+                                           int hidden, float eps, float w_offset, float* hist, long long hist_stride,
                                            int n_prev, const void* __restrict__ coef, int coef_dtype, bf16* __restrict__ low) {
   pdl_trigger();
   __shared__ float red[32];
@@ -265,7 +266,25 @@ __global__ void branch_norm_add_vec_kernel(float* __restrict__ h, const TA* __re
       for (int e = 0; e < 4; ++e) ss += av[k][e] * av[k][e];
     }
   }
-  ss = block_sum(ss, red);      // its barriers also publish cf
+  if (hist != nullptr) __syncthreads();      // cf
+  // the average's earlier terms wait for no norm: their loads run beside the reduction
+  float acc[VPT][4];
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int v = threadIdx.x + k * blockDim.x;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[k][e] = 0.f;
+    if (hist == nullptr || v >= nvec) continue;
+#pragma unroll 8
+    for (int j = 0; j < n_prev; ++j) {
+      float p[4];
+      load4(hist + (size_t)j * hist_stride + row + (size_t)v * 4, p);
+      const float c = cf[j];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[k][e] += c * p[e];
+    }
+  }
+  ss = block_sum(ss, red);
   const float inv = rsqrtf(ss / (float)hidden + eps);
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
@@ -277,18 +296,9 @@ __global__ void branch_norm_add_vec_kernel(float* __restrict__ h, const TA* __re
     for (int e = 0; e < 4; ++e) x[e] = hv[k][e] + av[k][e] * inv * (w_offset + wv[k][e]);
     if (hist != nullptr) {
       store4(hist + (size_t)n_prev * hist_stride + at, x);
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-      for (int j = 0; j < n_prev; ++j) {
-        float p[4];
-        load4(hist + (size_t)j * hist_stride + at, p);
-        const float c = cf[j];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[e] += c * p[e];
-      }
       const float c = cf[n_prev];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) x[e] = acc[e] + c * x[e];
+      for (int e = 0; e < 4; ++e) x[e] = acc[k][e] + c * x[e];
     }
     store4(h + at, x);
     if (low != nullptr) store4(low + at, x);
@@ -449,7 +459,7 @@ constexpr int kConvFewTokens = 128;
 constexpr int kConvMaxTaps = 8;
 template <typename TX, typename TO, int kTaps, int kRows>     // kTaps: 2, 4 or 8, at least the taps; kRows: rows a thread
 __global__ void __launch_bounds__(256) short_conv_vec_kernel(
-    TO* __restrict__ out, const TX* __restrict__ x, const void* __restrict__ w, int w_dtype, float* __restrict__ state,
+    TO* out, const TX* x, const void* __restrict__ w, int w_dtype, float* state,
     long long state_stride, const int* __restrict__ cu_seqlens, const int* __restrict__ token_req,
     const int* __restrict__ state_slots, const int* __restrict__ state_phase, int tokens, int channels, int taps, int add_input,
     int conv_blocks, long long x_stride, long long out_stride, int act, const float* __restrict__ in_bias,
@@ -468,13 +478,14 @@ __global__ void __launch_bounds__(256) short_conv_vec_kernel(
   if ((int)blockIdx.x >= conv_blocks) {
     // The blocks behind the filter's own: one per request, they leave the state as it stands after the step in the copy
     // that the step does not read (the filter's blocks read the other one, so the two kinds of block never meet).
-    pdl_wait();
     const int b = blockIdx.x - conv_blocks;
     const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start;
-    if (c >= channels || n <= 0 || token_req[start] < 0) return;   // a padding request of a recorded step owns no state
     const int phase = state_phase[b];
     const float* old = state + (size_t)state_slots[b] * state_stride + (size_t)phase * keep * channels;
     float* nx = state + (size_t)state_slots[b] * state_stride + (size_t)(1 - phase) * keep * channels;
+    const bool live = c < channels && n > 0 && token_req[start] >= 0;   // a padding request of a recorded step owns no state
+    pdl_wait();
+    if (!live) return;
     for (int k = 0; k < keep; ++k) {
       const int s = n + k - keep;
       float v[4];
@@ -494,6 +505,33 @@ __global__ void __launch_bounds__(256) short_conv_vec_kernel(
         for (int e = 0; e < 4; ++e) wt[j][e] = load_as_f32(w, w_dtype, (size_t)(c + e) * taps + keep - j);   // of the input j rows above
       }
   }
+  // What depends on no kernel of the step, before the wait: the requests of the rows and of the taps - 1 rows above them (a
+  // request's rows are consecutive, so a row's place in its portion shows in its neighbours' requests alone), and, where a
+  // thread has one row, the old state that this row needs.
+  const int t_end = min(tokens, t0 + kRows);
+  int reqs[kRows + kTaps - 1];
+#pragma unroll
+  for (int i = 0; i < kRows + kTaps - 1; ++i) {
+    const int r = t0 - (kTaps - 1) + i;
+    reqs[i] = (r >= 0 && r < t_end && r >= t0 - keep) ? token_req[r] : -2;
+  }
+  auto place = [&](int i) {      // rows of the same request directly above row i, counted up to taps - 1
+    int rel = 0;
+#pragma unroll
+    for (int j = 1; j < kTaps; ++j)
+      if (j <= keep && rel == j - 1 && reqs[i + kTaps - 1 - j] == reqs[i + kTaps - 1]) rel = j;
+    return rel;
+  };
+  float early[kRows == 1 ? kTaps : 1][4];      // early[j]: the state's row that stands j rows above this one
+  if (kRows == 1 && t0 < t_end && c < channels) {
+    const int req = reqs[kTaps - 1], rel = place(0);
+    if (req >= 0) {
+      const float* st = state + (size_t)state_slots[req] * state_stride + (size_t)state_phase[req] * keep * channels;
+#pragma unroll
+      for (int j = 1; j < kTaps; ++j)
+        if (j <= keep && j > rel) load4(st + (size_t)(keep + rel - j) * channels + c, early[kRows == 1 ? j : 0]);
+    }
+  }
   pdl_wait();
   if (c >= channels) return;
   // ring[i]: the input i + 1 rows above the current one
@@ -503,16 +541,7 @@ __global__ void __launch_bounds__(256) short_conv_vec_kernel(
     const int r = t0 - 1 - j;
     if (j < keep && r >= 0) load_in(x + (size_t)r * x_stride + c, ring[j]);
   }
-  const int t_end = min(tokens, t0 + kRows);
-  // The requests of the rows and of the taps - 1 rows above them, and the rows' inputs: all asked for before any is used.
-  // A request's rows are consecutive, so a row's place in its portion shows in its neighbours' requests alone.
-  int reqs[kRows + kTaps - 1];
-  float curs[kRows][4];
-#pragma unroll
-  for (int i = 0; i < kRows + kTaps - 1; ++i) {
-    const int r = t0 - (kTaps - 1) + i;
-    reqs[i] = (r >= 0 && r < t_end && r >= t0 - keep) ? token_req[r] : -2;
-  }
+  float curs[kRows][4];        // all asked for before any is used
 #pragma unroll
   for (int i = 0; i < kRows; ++i)
     if (t0 + i < t_end) load_in(x + (size_t)(t0 + i) * x_stride + c, curs[i]);
@@ -521,10 +550,7 @@ __global__ void __launch_bounds__(256) short_conv_vec_kernel(
     const int t = t0 + i;
     if (t >= t_end) break;
     const int req = reqs[i + kTaps - 1];
-    int rel = 0;                 // rows of the same request directly above, counted up to taps - 1
-#pragma unroll
-    for (int j = 1; j < kTaps; ++j)
-      if (j <= keep && rel == j - 1 && reqs[i + kTaps - 1 - j] == req) rel = j;
+    const int rel = place(i);
     // a portion's first rows read the copy of the request's state that is current in this step
     const float* st = (req >= 0 && rel < keep)
                           ? state + (size_t)state_slots[req] * state_stride + (size_t)state_phase[req] * keep * channels : nullptr;
@@ -544,6 +570,9 @@ __global__ void __launch_bounds__(256) short_conv_vec_kernel(
       } else if (rel - j >= 0) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) v[e] = ring[j - 1][e];
+      } else if (kRows == 1 && req >= 0) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = early[kRows == 1 ? j : 0][e];
       } else if (st) {
         load4(st + (size_t)(keep + rel - j) * channels + c, v);
       }

@@ -70,6 +70,9 @@ typedef __nv_bfloat16 bf16;
 // starts after that kernel has started. Keys and values of earlier steps lie behind that fence too.
 // A kernel launched without the attribute (oi_set_pdl(0), or after a library kernel) sees both
 // instructions as no-ops.
+// In a kernel that reads anything before its wait, what other kernels of the step write is not reached through __restrict__
+// pointers: such a pointer promises the compiler that nothing else changes what it reads, the wait included, and a load
+// behind the wait may then be moved up to join those before it.
 // ---------------------------------------------------------------------------------------------
 int oi_pdl_enabled();
 void oi_fence_next_launch();   // the next kernel launched through oi_launch gets plain stream order (once)

@@ -183,25 +183,29 @@ mingru_scan_kernel(TO* __restrict__ out, long long out_stride, const float* __re
 
 // the requests that bring one row
 template <typename TO, bool kFast>
-__global__ void mingru_step_kernel(TO* __restrict__ out, long long out_stride, const float* __restrict__ zug, long long stride,
-                                   int col_step, const float* __restrict__ bias, float* __restrict__ state, long long state_stride,
+__global__ void mingru_step_kernel(TO* out, long long out_stride, const float* zug, long long stride,
+                                   int col_step, const float* __restrict__ bias, float* state, long long state_stride,
                                    const int* __restrict__ cu_seqlens, const int* __restrict__ token_req,
                                    const int* __restrict__ state_slots, int channels) {
-  pdl_start();
+  pdl_trigger();
+  // the metadata, the biases and the old state depend on no kernel of the step: before the wait
   const int b = blockIdx.x, t = cu_seqlens[b];
-  if (cu_seqlens[b + 1] - t != 1) return;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
-  if (c >= channels) return;
+  const bool live = cu_seqlens[b + 1] - t == 1 && c < channels, padding = live && token_req[t] < 0;
+  float* st = state + (size_t)state_slots[b] * state_stride + c;
+  float old = 0.f, bz = 0.f, bx = 0.f;
+  if (live && !padding) old = *st, bz = bias[c], bx = bias[channels + c];
+  pdl_wait();
+  if (!live) return;
   TO* o = out + (size_t)t * out_stride + c;
-  if (token_req[t] < 0) {
+  if (padding) {
     *o = from_f32<TO>(0.f);
     return;
   }
   const float* p = zug + (size_t)t * stride + c;
-  float* st = state + (size_t)state_slots[b] * state_stride + c;
   float a, v;
-  keep_and_add<kFast>(p[0] + bias[c], p[col_step] + bias[channels + c], a, v);
-  const float S = a * *st + v;
+  keep_and_add<kFast>(p[0] + bz, p[col_step] + bx, a, v);
+  const float S = a * old + v;
   *st = S;
   *o = from_f32<TO>(S * silu_f<kFast>(p[2 * col_step]));
 }

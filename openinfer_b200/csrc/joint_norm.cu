@@ -85,9 +85,9 @@ struct JointArgs {
 };
 
 template <typename T, int V, int kKeep>
-__global__ void __launch_bounds__(256) joint_norm_half_store_kernel(T* __restrict__ qkv, T* __restrict__ k_cache, T* __restrict__ v_cache,
+__global__ void __launch_bounds__(256) joint_norm_half_store_kernel(T* qkv, T* __restrict__ k_cache, T* __restrict__ v_cache,
                                                                     const JointArgs p) {
-  pdl_start();
+  pdl_trigger();
   __shared__ float red[64];
   const int t = blockIdx.x, step = blockDim.x, hd = p.hd;
   T* row = qkv + (size_t)t * p.row_stride;
@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(256) joint_norm_half_store_kernel(T* __restric
   const int slot = p.slots[t];
   int pos = p.positions[t];
   pos = pos < 0 ? 0 : (p.rot_half > 0 && pos >= p.max_pos ? p.max_pos - 1 : pos);      // admission bounds positions
+  pdl_wait();            // (the step's metadata before it)
   // the columns of item i: c and c + gap of the row (k heads lie behind the q heads)
   auto column = [&](int i, int& gap) {
     const int head = i / per, n = i - head * per;

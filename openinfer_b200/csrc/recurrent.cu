@@ -304,14 +304,17 @@ __device__ __forceinline__ void load_channels(float (&dst)[R], const float* __re
 
 template <int kMode, int kLanes, int R, bool kVec4>
 __global__ void __launch_bounds__(kThreads) recurrent_scan_kernel(ScanArgs a, int chunk) {
-  pdl_wait();    // no early trigger: the blocks of the kernel behind this one would wait on the SMs this latency-bound loop needs
+  // (no early trigger: the blocks of the kernel behind this one would wait on the SMs this latency-bound loop needs)
   extern __shared__ __align__(16) float stage[];   // two buffers of [chunk][rec] records, then [chunk][cols] values
   constexpr bool kGates = kMode == kMatrixMemory;
   constexpr int kE = 2, kCols = kE * kThreads / kLanes;
   static_assert(kLanes >= 8, "a lane ends up with one column's and one row's sum");
   const int b = blockIdx.x, h = blockIdx.y;
   const int start = a.cu_seqlens[b], n_rows = a.cu_seqlens[b + 1] - start;
-  if (n_rows <= 0 || a.token_req[start] < 0) return;    // a padding request of a recorded step owns no state
+  if (n_rows <= 0 || a.token_req[start] < 0) {    // a padding request of a recorded step owns no state
+    pdl_wait();
+    return;
+  }
   const int j = threadIdx.x % kLanes, pair = threadIdx.x / kLanes;
   const int c0 = blockIdx.z * kCols + kE * pair;
   const int D = a.D, V = a.V, rec = a.rec;
@@ -426,6 +429,7 @@ __global__ void __launch_bounds__(kThreads) recurrent_scan_kernel(ScanArgs a, in
       a.out[(size_t)(first_row + my_row) * a.ld_out + (size_t)h * V + c0 + my_col] = kGates ? num[0] / (fmaxf(fabsf(den[0]), bound) + 1e-6f) : num[0];
     }
   };
+  pdl_wait();    // the old state's copy is the step before's: only the records and values are this step's
   request(0, 0);
   int turn = 0;
   for (int t0 = 0; t0 < n_rows; t0 += chunk, turn ^= 1) {      // chunk: a multiple of four
@@ -465,13 +469,15 @@ __global__ void __launch_bounds__(kThreads) recurrent_scan_kernel(ScanArgs a, in
 // up to 1,500 rows, 8 heads of 128 keys and values, took 750 us, and this 382 us (440 us with chunks of 8 rows, 608 us with 8 lanes).
 template <int kLanes, int R, bool kVec4>
 __global__ void __launch_bounds__(kThreads) delta_channel_scan_kernel(ScanArgs a, int chunk) {
-  pdl_wait();    // (no early trigger, as above)
   extern __shared__ __align__(16) float stage[];      // two buffers of [chunk / 4] runs, then [chunk][cols] values
   constexpr int kE = 2, kCols = kE * kThreads / kLanes;
   static_assert(kLanes >= 8, "a lane ends up with one column's and one row's sums");
   const int b = blockIdx.x, h = blockIdx.y;
   const int start = a.cu_seqlens[b], n_rows = a.cu_seqlens[b + 1] - start;
-  if (n_rows <= 0 || a.token_req[start] < 0) return;
+  if (n_rows <= 0 || a.token_req[start] < 0) {
+    pdl_wait();
+    return;
+  }
   const int lane = threadIdx.x & 31, j = threadIdx.x % kLanes, pair = threadIdx.x / kLanes;
   const int c0 = blockIdx.z * kCols + kE * pair;
   const int D = a.D, V = a.V, D4 = padded4(D), row = run_row(D), full_run = 4 * row + D4;
@@ -592,6 +598,7 @@ __global__ void __launch_bounds__(kThreads) delta_channel_scan_kernel(ScanArgs a
         for (int i = 0; i < R; ++i) C[e][i] += k[i] * d[e][u];
     }
   };
+  pdl_wait();    // the old state's copy is the step before's: only the records and values are this step's
   request(0, 0);
   int turn = 0;
   for (int t0 = 0; t0 < n_rows; t0 += chunk, turn ^= 1) {      // chunk: a multiple of four, so that runs do not straddle it
@@ -627,13 +634,15 @@ __global__ void __launch_bounds__(kThreads) delta_channel_scan_kernel(ScanArgs a
 // kind) has its one.
 template <int kLanes, int R, bool kVec4>
 __global__ void __launch_bounds__(kThreads) delta_head_scan_kernel(ScanArgs a, int chunk) {
-  pdl_wait();    // (no early trigger, as above)
   extern __shared__ __align__(16) float stage[];
   constexpr int kE = 2;                             // columns a lane
   constexpr int kCols = kE * kThreads / kLanes, kRowStep = kLanes / (4 * kE), kKindStep = kLanes / (8 * kE);
   const int b = blockIdx.x, h = blockIdx.y;
   const int start = a.cu_seqlens[b], n_rows = a.cu_seqlens[b + 1] - start;
-  if (n_rows <= 0 || a.token_req[start] < 0) return;
+  if (n_rows <= 0 || a.token_req[start] < 0) {
+    pdl_wait();
+    return;
+  }
   const int lane = threadIdx.x & 31, j = threadIdx.x % kLanes, pair = threadIdx.x / kLanes;
   const int c0 = blockIdx.z * kCols + kE * pair;
   const int D = a.D, V = a.V, rec = a.rec, at = delta_scalars_at(D);
@@ -666,6 +675,7 @@ __global__ void __launch_bounds__(kThreads) delta_head_scan_kernel(ScanArgs a, i
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
+  pdl_wait();    // the old state's copy is the step before's: only the records and values are this step's
   request(0, 0);
   int turn = 0;
   for (int t0 = 0; t0 < n_rows; t0 += chunk, turn ^= 1) {      // chunk: a multiple of four, so that runs do not straddle it
@@ -868,6 +878,10 @@ OI_API int oi_recurrent_scan(int mode, const float* qkv, long long ld_qkv, int q
   else if (mode == kDeltaHeadDecay) oi_launch(delta_head_prepare_kernel, (warps + 3) / 4, 128, 0, s, a);
   else oi_launch(delta_channel_prepare_kernel, (warps + 3) / 4, 128, 0, s, a);
   OI_CHECK_LAUNCH();
+  // Requests of several rows in plain stream order: launched early, the few long-lived blocks would be packed onto the SMs that
+  // the kernel before frees first and share their issue slots (measured 2.1 against 0.9 ms for 2,048 rows). Single rows have no
+  // such loop: launched early they fetch the old state while the records are formed.
+  const bool single = tokens == requests;
   if (mode == kDeltaHeadDecay) {
     const int rows = D <= 128 ? 16 : (D <= 256 ? 8 : 4);       // per buffer: two buffers of at most 19 KB
 #define OI_DELTA_HEAD(LANES, REGS)                                                                                          \
@@ -875,7 +889,7 @@ OI_API int oi_recurrent_scan(int mode, const float* qkv, long long ld_qkv, int q
     constexpr int cols = 2 * kThreads / LANES;                                                                              \
     const dim3 grid(requests, H, (V + cols - 1) / cols);                                                                    \
     const size_t smem = 2 * (size_t)rows * (a.rec + cols) * sizeof(float);                                                  \
-    oi_fence_next_launch();      /* plain stream order, as below */                                                         \
+    if (!single) oi_fence_next_launch();                                                                                    \
     if (D % 4 == 0) oi_launch(delta_head_scan_kernel<LANES, REGS, true>, grid, kThreads, smem, s, a, rows);                 \
     else oi_launch(delta_head_scan_kernel<LANES, REGS, false>, grid, kThreads, smem, s, a, rows);                           \
   } while (0)
@@ -898,7 +912,7 @@ OI_API int oi_recurrent_scan(int mode, const float* qkv, long long ld_qkv, int q
     constexpr int cols = 2 * kThreads / LANES;                                                                              \
     const dim3 grid(requests, H, (V + cols - 1) / cols);                                                                    \
     const size_t smem = 2 * ((size_t)(rows / 4) * (4 * run_row(D) + padded4(D)) + rows * cols) * sizeof(float);             \
-    oi_fence_next_launch();      /* plain stream order, as below */                                                         \
+    if (!single) oi_fence_next_launch();                                                                                    \
     auto kernel = D % 4 == 0 ? delta_channel_scan_kernel<LANES, REGS, true> : delta_channel_scan_kernel<LANES, REGS, false>; \
     if (smem > 48 * 1024) OI_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
     oi_launch(kernel, grid, kThreads, smem, s, a, rows);                                                                    \
@@ -920,9 +934,7 @@ OI_API int oi_recurrent_scan(int mode, const float* qkv, long long ld_qkv, int q
     constexpr int cols = 2 * kThreads / LANES;                                                                          \
     const dim3 grid(requests, H, (V + cols - 1) / cols);                                                                \
     const size_t smem = 2 * (size_t)chunk * (a.rec + cols) * sizeof(float);                                                 \
-    /* plain stream order: launched early, the few long-lived blocks would be packed onto the SMs that the kernel */     \
-    /* before frees first and share their issue slots (measured 2.1 against 0.9 ms for 2,048 rows) */                   \
-    oi_fence_next_launch();                                                                                              \
+    if (!single) oi_fence_next_launch();                                                                                \
     auto kernel = D % 4 == 0 ? recurrent_scan_kernel<MODE, LANES, REGS, true> : recurrent_scan_kernel<MODE, LANES, REGS, false>; \
     if (smem > 48 * 1024) OI_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
     oi_launch(kernel, grid, kThreads, smem, s, a, chunk);                                                               \

@@ -100,18 +100,19 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
 // kKeep: eights of q | k a thread keeps in registers between the sum and the turn (0: they are read again)
 template <typename T, int kKeep>
 __global__ void __launch_bounds__(kThreads)
-joint_norm_rope_store_kernel(T* __restrict__ proj, long long row_stride, int nq, int nkv, int hd, int qk_dim, int k_off, int v_off,
+joint_norm_rope_store_kernel(T* proj, long long row_stride, int nq, int nkv, int hd, int qk_dim, int k_off, int v_off,
                              const float* __restrict__ q_w, const float* __restrict__ k_w, float eps,
                              const float* __restrict__ cos_tab, const float* __restrict__ sin_tab, int rot_half, int max_pos,
                              const int* __restrict__ positions, const int* __restrict__ slots, T* __restrict__ k_cache,
                              T* __restrict__ v_cache, long long page_stride, int page_size) {
-  pdl_start();
+  pdl_trigger();
   __shared__ float red[64];
   const int t = blockIdx.x, step = blockDim.x;
   T* row = proj + (size_t)t * row_stride;
   const int q8 = nq * hd / 8, k8 = nkv * hd / 8;
-  const int slot = slots[t];
+  const int slot = slots[t];      // (the step's metadata: before the wait)
   int pos = positions[t];
+  pdl_wait();
   float keep[kKeep ? kKeep : 1][8];
   auto source = [&](int i) { return i < q8 ? row + (size_t)i * 8 : row + k_off + (size_t)(i - q8) * 8; };
   float q_inv = 1.f, k_inv = 1.f;
