@@ -126,6 +126,10 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (threadIdx.x == 0) atomicCAS(&g_stream_error, 0, 9);
   }
 
+  if (threadIdx.x == 64) {      // x's map is first used behind the wait: its descriptor is here by then
+    tc::prefetch_map(&map_w);
+    tc::prefetch_map(&map_x);
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       tc::mbar_init(full_bar(s), 1);
@@ -264,7 +268,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (c0 == 0 && csize > 1) tc::cluster_wait();       // phase 0: every CTA of the cluster runs
         float* dst = (csize > 1 ? cg::this_cluster().map_shared_rank(recv, owner) : recv) + (size_t)(rank * BN + c0) * share + local;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) dst[e * share] = __uint_as_float(v[e]);
+        for (int e = 0; e < 16; ++e)
+          if (c0 + e < M) dst[e * share] = __uint_as_float(v[e]);
       }
     }
   }

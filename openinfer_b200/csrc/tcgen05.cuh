@@ -50,6 +50,10 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatil
   return false;
 }
 
+// the descriptor of a map that a later copy uses: its fetch from memory is on the way before that copy is issued
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map, int c0, int c1, unsigned bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
