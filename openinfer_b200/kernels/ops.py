@@ -243,7 +243,7 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor,
                       page_stride: int, page_size: int, block_table: torch.Tensor, token_req: torch.Tensor,
                       positions: torch.Tensor, nq: int, nkv: int, hd: int, scale: float,
                       window: Optional[int] = None, mods=None) -> torch.Tensor:
-    """Paged causal attention, one warp per (token, head). ``q`` is [tokens, >= nq*hd] with
+    """Paged causal attention, any shape. ``q`` is [tokens, >= nq*hd] with
     any row stride; ``out`` is [tokens, nq*hd]; ``block_table`` is int32 [requests, max_pages]; ``mods`` a
     ``native.ScoreMods`` (sink, slopes, cap, query temperature) or None."""
     import ctypes

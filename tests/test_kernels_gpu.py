@@ -1367,3 +1367,55 @@ def test_recurrent_scan_runs_of_rows(mode, D, V):
             assert (got[: D * V].view(V, D) - C).abs().max() < 3e-5 * (1 + C.abs().max())
             if memory:
                 assert (got[D * V: D * V + D] - n).abs().max() < 3e-5 * (1 + n.abs().max()) and abs(got[-1] - m) < 3e-5 * (1 + abs(m))
+
+
+# ------------------------------------------------------------------------------------------------ one block a row, its row in registers
+@pytest.mark.parametrize("hidden", [4, 36, 2048, 2052, 4096, 4100, 8192, 8196, 101])
+@pytest.mark.parametrize("center", [False, True])
+@pytest.mark.parametrize("src,dst,wt", [("float32", "bfloat16", "bfloat16"), ("bfloat16", "float32", "float32"), ("float32", "float32", "bfloat16")])
+def test_norm_cast_widths(hidden, center, src, dst, wt):
+    """One, two and four fours a thread, the widths behind each limit, and widths that are no whole fours."""
+    from openinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(hidden)
+    x = (torch.randn(7, hidden, generator=g) * 3 + 1).to(getattr(torch, src))
+    w = torch.randn(hidden, generator=g).to(getattr(torch, wt))
+    idx = torch.tensor([6, 0, 3], dtype=torch.int32)
+    out = torch.empty(3, hidden, dtype=getattr(torch, dst), device=DEV)
+    ops.rmsnorm_cast(out, x.to(DEV), w.to(DEV), 1e-5, row_idx=idx.to(DEV), weight_offset=1.0, center=center)
+    v = x[idx.long()].double()
+    v = v - v.mean(-1, keepdim=True) if center else v
+    ref = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5) * (1.0 + w.double())
+    # float32 sums of up to 8,196 terms and a mean taken off: some 2^-18; a rounding to bfloat16, 8 significant bits: half a
+    # unit of the last place is at most 2^-8 of the value
+    step = 2.0 ** -8 if dst == "bfloat16" else 0.0
+    assert ((out.cpu().double() - ref).abs() <= ref.abs() * (step + 2.0 ** -18) + 2.0 ** -18 * (1.0 + w.double().abs())).all()
+
+
+@pytest.mark.parametrize("S,W", [(1, 4), (2, 36), (2, 2048), (3, 2052), (4, 4096), (4, 4100), (5, 2048), (2, 101)])
+@pytest.mark.parametrize("dst", ["float32", "bfloat16"])
+def test_hyper_step_widths(S, W, dst):
+    """A thread keeps one or two fours of the combined row; widths behind each limit, no whole fours, more than four streams."""
+    from openinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(S * W)
+    X, y = torch.randn(3, S, W, generator=g), torch.randn(3, W, generator=g)
+    M, b, a, w = torch.randn(S, S, generator=g), torch.randn(S, generator=g), torch.randn(S, generator=g), torch.randn(W, generator=g)
+    Xd, out = X.to(DEV), torch.empty(3, W, dtype=getattr(torch, dst), device=DEV)
+    ops.hyper_step(Xd, y=y.to(DEV), mix=M.to(DEV), b_out=b.to(DEV), a_in=a.to(DEV), norm_w=w.to(DEV), eps=1e-5, weight_offset=1.0, out=out)
+    new = torch.einsum("sr,tsw->trw", M.double(), X.double()) + b.double()[None, :, None] * y.double()[:, None]
+    u = torch.einsum("s,tsw->tw", a.double(), new)
+    ref = u * torch.rsqrt(u.pow(2).mean(-1, keepdim=True) + 1e-5) * (1.0 + w.double())
+    # sums of at most 6 and then 5 products of numbers below some 5: 2^-24 of 5 x 25 each; the norm's sums as above
+    assert (Xd.cpu().double() - new).abs().max() <= 2.0 ** -17
+    step = 2.0 ** -8 if dst == "bfloat16" else 0.0
+    slack = 2.0 ** -14 * (1.0 + w.double().abs()) / u.pow(2).mean(-1, keepdim=True).sqrt().clamp(max=1.0)
+    assert ((out.cpu().double() - ref).abs() <= ref.abs() * (step + 2.0 ** -18) + slack).all()
+
+
+@pytest.mark.parametrize("hidden", [4, 132, 2048, 2056, 6])
+def test_embedding_widened(hidden):
+    from openinfer_b200.kernels import ops
+    table = torch.randn(19, hidden, device=DEV).to(torch.bfloat16)
+    ids = torch.tensor([0, 18, 7, 7, 3], dtype=torch.int32, device=DEV)
+    out = torch.empty(5, hidden, device=DEV)
+    ops.embedding(out, table, ids)
+    assert torch.equal(out, table[ids.long()].float())
