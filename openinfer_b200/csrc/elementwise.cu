@@ -177,7 +177,7 @@ __global__ void rmsnorm_kernel(T* __restrict__ out, T* __restrict__ x, const T* 
 // bfloat16 rows whose length is a multiple of 8 and a bfloat16 weight: every thread moves whole
 // 16-byte vectors, all loads (row, residual, weight) are issued before anything waits on them.
 template <int VPT>
-__global__ void rmsnorm_bf16_vec_kernel(bf16* __restrict__ out, bf16* __restrict__ x, const bf16* __restrict__ delta,
+__global__ void rmsnorm_bf16_vec_kernel(bf16* out, bf16* x, const bf16* delta,
                                         const bf16* __restrict__ w, const int* __restrict__ row_idx, int hidden,
                                         float eps, float w_offset) {
   pdl_trigger();
