@@ -15,12 +15,13 @@
 //                          then the down projection, each row written to its pair's place
 //   4. moe_combine_kernel  out[row] = sum_j weight[row, j] * y[row * top + j], j ascending
 //
-// Steps of few rows (at most two pairs an expert on average) skip 2 and stream every chosen expert's weights through the
-// tensor cores once (moe_stream.cu). Larger steps take tcgen05 tiles of 256 places (gemm_tcgen05.cu, over rows that
-// moe_gather_kernel has sorted): a tile of a few places costs what its expert's weights cost to read, so this holds from
-// the smallest such step on. Both want bfloat16 rows that TMA can read; other rows go pair by pair (moe_gemv_kernel: a
-// warp per output row) or by tiles of 32 places on the ordinary pipes. In batch-invariant mode the tiles of 32 and
-// 128 places on mma.sync take steps of any size, with the same sums.
+// Steps of few rows (at most two pairs an expert on average) skip 2 and read every chosen expert's weights once for up to four
+// pairs, on the ordinary pipes (moe_few_rows_kernel; rows that cannot be read 16 bytes at a time go pair by pair,
+// moe_gemv_kernel). Larger steps of bfloat16 rows that TMA can read take tcgen05 tiles of 256 places (gemm_tcgen05.cu, over
+// rows that moe_gather_kernel has sorted; their sums are bit for bit those of the mma.sync tiles): a tile of a few places costs
+// what its expert's weights cost to read, so this holds from the smallest such step on. Other rows go by tiles of 32 places on
+// the ordinary pipes. In batch-invariant mode the tiles of 32 and 128 places on mma.sync take steps of any size, with the
+// same sums.
 // Everything a step needs is found on the device (no sizes travel back to the host), so a step of single tokens can be
 // recorded and replayed. A row's sums are formed in the same order whatever else shares its tile.
 #include <type_traits>
@@ -606,63 +607,232 @@ __global__ void moe_gather_kernel(bf16* __restrict__ dst, const bf16* __restrict
   }
 }
 
-// The same two products for steps of few rows (at most two pairs an expert on average): one block per (pair, 16 output
-// rows), a warp per output row at a time, the pair's input row in shared memory as float32, the expert's rows read 16 bytes
-// at a time. No grouping is needed: pair p reads row p / a_div (a_div 0: row p) and writes row p.
+// The same two products for steps of few rows (at most two pairs an expert on average, kFewPairs in all): no grouping is needed. Pair
+// p reads row p / a_div (a_div 0: row p) and writes row p. Every sum is a warp's, in float32 on the ordinary pipes: lane l adds
+// the products of 16 bytes of the row, of the 16 bytes 32 places further on, and so on, and the lanes' sums are added as a tree.
+//
+// Measured on B200 (us for both products and the sum, inside a graph, 16 experts, two a row; a block per (pair, 16 rows) with loads where
+// they are used / products on tcgen05 that read every expert once / this): 2,048 x 1,536: 1 row 48 / 17 / 15, 4 rows 51 / 30 / 33, 8 rows
+// 76 / 38 / 49, 16 rows 111 / 57 / 69; 1,024 x 768: 25 / 13 / 12, 26 / 17 / 19, 27 / 20 / 26, 39 / 25 / 35. The tensor cores' sums are
+// shorter of precision: against 64 bits the result of 8 rows was off by 1.7e-4, this is off by 1.7e-5 (both mostly activations
+// that round to the other bfloat16), so they are not taken. Bound by latency and issue slots (0.44 instructions a clock of a
+// scheduler), above 2 rows at some 4 of the 6.5 TB/s. 256 threads and two blocks an SM: with 384 or 512 an SM 53 us for 8 rows; the
+// launch of the second product ahead of the first one's end: 53 -> 49; shares by what an expert costs: 16 rows 87 -> 73.
+constexpr int kFewPairs = 64, kFewThreads = 256, kFewBlocks = 2, kFewStages = 5;
+constexpr int kFewStage = 4 * 32;                                    // 16-byte words of a warp's stage: four rows, a word a lane
+constexpr int kFewRing = kFewThreads / 32 * kFewStages * kFewStage * 16;
+constexpr int kFewInputs = 24 * 1024;                                // bytes of input rows, where one takes no more
+
+__device__ __forceinline__ void few_cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// 16 bytes as floats, an instruction a number
+__device__ __forceinline__ void few_unpack(const uint4& v, float (&o)[8]) {
+  const unsigned u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[2 * i] = __uint_as_float(u[i] << 16), o[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+}
+__device__ __forceinline__ void few_unpack(const uint4& v, float (&o)[4]) {
+  o[0] = __uint_as_float(v.x), o[1] = __uint_as_float(v.y), o[2] = __uint_as_float(v.z), o[3] = __uint_as_float(v.w);
+}
+
+template <typename T, typename TO>
+struct FewRows {
+  const T* A;
+  long long lda;
+  int a_div;
+  const T* We;          // the expert's rows
+  TO* out;
+  long long ld_out;
+  int n_begin, n_end, N, K;
+  float limit;
+  int act;
+  bool x_vec;           // rows of A start on 16 bytes
+};
+
+// Output rows [n_begin, n_end) for P pairs that chose the expert. A warp takes four weight rows at a time (with the activation two
+// gate rows and their up rows), its ring of stages always ahead of it, from before the input rows are there and across its output
+// rows. A lane reads what it has fetched itself: no barrier, only its own copies to wait for.
+template <int P, bool kGlu, typename T, typename TO>
+__device__ __forceinline__ void few_rows_product(const FewRows<T, TO>& f, uint4* ring, T* xs, const int* pair_of, bool wait) {
+  constexpr int kVec = 16 / (int)sizeof(T), kOut = kGlu ? 2 : 4, kWarpStep = kFewThreads / 32 * kOut, kStep = 32 * kVec;
+  const int lane = threadIdx.x & 31, K = f.K;
+  int n = f.n_begin + (int)(threadIdx.x >> 5) * kOut, k = lane * kVec, slot = 0;
+  int n_ahead = n, k_ahead = k, slot_ahead = 0;
+  const T* src[4];
+  auto rows_of = [&]() {               // (rows beyond the last read that one again and are not stored)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int row = kGlu ? min(n_ahead + (q >> 1), f.n_end - 1) + (q & 1) * f.N : min(n_ahead + q, f.n_end - 1);
+      src[q] = f.We + (size_t)row * K;
+    }
+  };
+  rows_of();
+  ring += lane;
+  auto fetch = [&]() {
+    if (n_ahead < f.n_end && k_ahead < K) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) few_cp16(ring + slot_ahead + q * 32, src[q] + k_ahead);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    k_ahead += kStep;
+    if (k_ahead - lane * kVec >= K) k_ahead = lane * kVec, n_ahead += kWarpStep, rows_of();
+    slot_ahead = slot_ahead == (kFewStages - 1) * kFewStage ? 0 : slot_ahead + kFewStage;
+  };
+#pragma unroll
+  for (int s = 0; s < kFewStages - 1; ++s) fetch();
+  if (wait) pdl_wait();
+  for (int j = 0; j < P; ++j) {
+    const T* xr = f.A + (size_t)(f.a_div > 0 ? pair_of[j] / f.a_div : pair_of[j]) * f.lda;
+    T* to = xs + j * K;
+    if (f.x_vec)
+      for (int i = threadIdx.x * kVec; i < K; i += kFewThreads * kVec) *reinterpret_cast<uint4*>(to + i) = *reinterpret_cast<const uint4*>(xr + i);
+    else
+      for (int i = threadIdx.x; i < K; i += kFewThreads) to[i] = xr[i];
+  }
+  __syncthreads();
+  float sum[P][4] = {};
+  while (n < f.n_end) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kFewStages - 2) : "memory");
+    uint4 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = ring[slot + q * 32];
+    fetch();                            // into the slot that was read in the turn before
+    if (k < K) {
+      float w[4][kVec];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) few_unpack(v[q], w[q]);
+#pragma unroll
+      for (int j = 0; j < P; ++j) {
+        float x[kVec];
+        few_unpack(*reinterpret_cast<const uint4*>(xs + j * K + k), x);
+#pragma unroll
+        for (int e = 0; e < kVec; ++e)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) sum[j][q] = fmaf(w[q][e], x[e], sum[j][q]);
+      }
+    }
+    slot = slot == (kFewStages - 1) * kFewStage ? 0 : slot + kFewStage;
+    k += kStep;
+    if (k - lane * kVec < K) continue;
+    // the sums over the lanes, as warp_sum adds them; the two halves (with no activation the quarters) of the warp end up with
+    // different output rows
+    const bool up = (lane & 16) != 0, odd = (lane & 8) != 0;
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      float a = up ? sum[j][2] : sum[j][0], b = up ? sum[j][3] : sum[j][1];
+      a += __shfl_xor_sync(0xffffffffu, up ? sum[j][0] : sum[j][2], 16);
+      b += __shfl_xor_sync(0xffffffffu, up ? sum[j][1] : sum[j][3], 16);
+      if (!kGlu) a = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+      for (int o = kGlu ? 8 : 4; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (kGlu) b += __shfl_xor_sync(0xffffffffu, b, o);
+      }
+      const int at = n + (kGlu ? lane / 16 : lane / 8);
+      if (lane % (kGlu ? 16 : 8) == 0 && at < f.n_end)
+        f.out[(size_t)pair_of[j] * f.ld_out + at] = from_f32<TO>(kGlu ? glu_act<false>(a, b, f.act, f.limit) : a);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sum[j][q] = 0.f;
+    }
+    n += kWarpStep, k = lane * kVec;
+  }
+}
+
+// The chosen experts' output rows are shared out evenly among the blocks (as many as the SMs hold at once), an expert's counted with
+// the passes over its weights and the pairs that chose it; up to `at_once` pairs share a pass, their input rows in shared memory.
+template <typename T, typename TO, bool kGlu>
+__global__ void __launch_bounds__(kFewThreads, kFewBlocks) moe_few_rows_kernel(
+    const T* A, long long lda, int a_div, const T* __restrict__ Wt, long long w_expert_stride, TO* out, long long ld_out,
+    const int* __restrict__ ids, int pairs, int E, int N, int K, float limit, int act, int at_once, int x_vec) {
+  // The second product follows the first in the stream, and the first lets it start only when it has itself seen the choices:
+  // they, and the weights, may be read before the wait for the first product's results.
+  if (kGlu) pdl_wait();
+  pdl_trigger();
+  bool waited = kGlu;
+  extern __shared__ __align__(16) uint4 few_smem[];       // the warps' rings, then the input rows
+  uint4* const ring = few_smem + (threadIdx.x >> 5) * (kFewStages * kFewStage);
+  T* const xs = reinterpret_cast<T*>(few_smem + kFewRing / 16);
+  __shared__ int pair_of[kFewPairs], expert_of[kFewPairs], count_of[kFewPairs], s_chosen;
+  constexpr int kOut = kGlu ? 2 : 4;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1;
+  int id0 = -1, id1 = -1;
+  if (threadIdx.x < 32) {
+    // the choices of pairs lane, lane + 32 (one behind the experts stands for the row itself and counts as none), and the
+    // experts that were chosen, in order of first choice, with the number of pairs that chose them
+    if (lane < pairs) id0 = ids[lane];
+    if (lane + 32 < pairs) id1 = ids[lane + 32];
+    if (id0 >= E) id0 = -1;
+    if (id1 >= E) id1 = -1;
+    const unsigned same0 = __match_any_sync(0xffffffffu, id0);
+    int count0 = __popc(same0);
+    const bool first0 = id0 >= 0 && __ffs(same0) - 1 == lane;
+    const unsigned f0 = __ballot_sync(0xffffffffu, first0);
+    unsigned f1 = 0;
+    if (pairs > 32) {
+      bool again = false;        // id1 was chosen in the lower half
+      for (int i = 0; i < 32; ++i) {
+        again |= __shfl_sync(0xffffffffu, id0, i) == id1;
+        count0 += __shfl_sync(0xffffffffu, id1, i) == id0;
+      }
+      const unsigned same1 = __match_any_sync(0xffffffffu, id1);
+      const bool first1 = id1 >= 0 && !again && __ffs(same1) - 1 == lane;
+      f1 = __ballot_sync(0xffffffffu, first1);
+      const int z = __popc(f0) + __popc(f1 & below);
+      if (first1) expert_of[z] = id1, count_of[z] = __popc(same1);
+    }
+    if (first0) expert_of[__popc(f0 & below)] = id0, count_of[__popc(f0 & below)] = count0;
+    if (lane == 0) s_chosen = __popc(f0) + __popc(f1);
+  }
+  __syncthreads();
+  const int chosen = s_chosen, units = (N + kOut - 1) / kOut;      // units of kOut output rows
+  auto cost_of = [&](int count) { return (count + at_once - 1) / at_once + count; };
+  int all = 0;
+  for (int z = 0; z < chosen; ++z) all += units * cost_of(count_of[z]);
+  const int lo = (int)((long long)all * blockIdx.x / gridDim.x), hi = (int)((long long)all * (blockIdx.x + 1) / gridDim.x);
+  for (int z = 0, here = 0; z < chosen && here < hi; ++z) {
+    const int count = count_of[z], cost = cost_of(count), e = expert_of[z], begin = here;
+    here += units * cost;
+    // the units that begin in [lo, hi)
+    const int first = lo > begin ? (lo - begin + cost - 1) / cost : 0, last = hi < here ? (hi - begin + cost - 1) / cost : units;
+    if (first >= last) continue;
+    if (threadIdx.x < 32) {
+      // every pair that chose it, a row's second choice of the same expert too
+      const unsigned m0 = __ballot_sync(0xffffffffu, id0 == e), m1 = __ballot_sync(0xffffffffu, id1 == e);
+      if (id0 == e) pair_of[__popc(m0 & below)] = lane;
+      if (id1 == e) pair_of[__popc(m0) + __popc(m1 & below)] = lane + 32;
+    }
+    __syncthreads();
+    const FewRows<T, TO> f = {A, lda, a_div, Wt + (size_t)e * w_expert_stride, out, ld_out, first * kOut, min(N, last * kOut), N, K, limit, act, x_vec != 0};
+    for (int c = 0; c < count; c += at_once) {
+      const int np = min(at_once, count - c);
+      if (np == 1) few_rows_product<1, kGlu>(f, ring, xs, pair_of + c, !waited);
+      else if (np == 2) few_rows_product<2, kGlu>(f, ring, xs, pair_of + c, !waited);
+      else if (np == 3) few_rows_product<3, kGlu>(f, ring, xs, pair_of + c, !waited);
+      else few_rows_product<4, kGlu>(f, ring, xs, pair_of + c, !waited);
+      waited = true;
+      __syncthreads();        // everybody is through with the rows, and with the list
+    }
+  }
+  if (!waited) pdl_wait();
+}
+
+// Any alignment and any K: one block per (pair, 16 output rows), a warp per output row, its input row in shared memory.
 template <typename T, typename TO, bool kGlu>
 __global__ void __launch_bounds__(128) moe_gemv_kernel(const T* __restrict__ A, long long lda, int a_div, const T* __restrict__ Wt,
                                                        long long w_expert_stride, TO* __restrict__ out, long long ld_out,
                                                        const int* __restrict__ ids, int E, int N, int K, float limit, int act) {
-  pdl_wait();    // no early trigger: waiting blocks of the next kernel would share the SMs with this product
+  pdl_wait();    // (no early trigger, as above)
   extern __shared__ __align__(16) float xs[];
-  constexpr int kVec = 16 / (int)sizeof(T), kRows = 16;
+  constexpr int kRows = 16;
   if (ids[blockIdx.x] >= E) return;      // a choice that stands for the row itself
   const int p = blockIdx.x, lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   const T* xr = A + (size_t)(a_div > 0 ? p / a_div : p) * lda;
   for (int k = threadIdx.x; k < K; k += blockDim.x) xs[k] = to_f32(xr[k]);
   __syncthreads();
   const T* We = Wt + (size_t)ids[p] * w_expert_stride;
-  const bool vec = K % kVec == 0 && ((uintptr_t)We % 16 == 0);
   const int n_end = min(N, (int)(blockIdx.y + 1) * kRows);
-  if (vec) {
-    // two output rows of the warp at a time, two steps along K unrolled: eight 16-byte loads in flight a lane (a row beyond
-    // the block's last reads that one again and is not stored)
-    for (int n = blockIdx.y * kRows + wi; n < n_end; n += 8) {
-      const int n1 = n + 4 < n_end ? n + 4 : n;
-      const T* wg0 = We + (size_t)n * K;
-      const T* wg1 = We + (size_t)n1 * K;
-      const T* wu0 = wg0 + (size_t)N * K;
-      const T* wu1 = wg1 + (size_t)N * K;
-      float g0 = 0.f, u0 = 0.f, g1 = 0.f, u1 = 0.f;
-#pragma unroll 2
-      for (int k = lane * kVec; k < K; k += 32 * kVec) {
-        T a0[kVec], b0[kVec], a1[kVec], b1[kVec];
-        *reinterpret_cast<uint4*>(a0) = *reinterpret_cast<const uint4*>(wg0 + k);
-        *reinterpret_cast<uint4*>(a1) = *reinterpret_cast<const uint4*>(wg1 + k);
-        if (kGlu) {
-          *reinterpret_cast<uint4*>(b0) = *reinterpret_cast<const uint4*>(wu0 + k);
-          *reinterpret_cast<uint4*>(b1) = *reinterpret_cast<const uint4*>(wu1 + k);
-        }
-#pragma unroll
-        for (int e = 0; e < kVec; ++e) {
-          const float xv = xs[k + e];
-          g0 += to_f32(a0[e]) * xv;
-          g1 += to_f32(a1[e]) * xv;
-          if (kGlu) {
-            u0 += to_f32(b0[e]) * xv;
-            u1 += to_f32(b1[e]) * xv;
-          }
-        }
-      }
-      g0 = warp_sum(g0), g1 = warp_sum(g1);
-      if (kGlu) u0 = warp_sum(u0), u1 = warp_sum(u1);
-      if (lane == 0) {
-        out[(size_t)p * ld_out + n] = from_f32<TO>(kGlu ? glu_act<false>(g0, u0, act, limit) : g0);
-        if (n1 != n) out[(size_t)p * ld_out + n1] = from_f32<TO>(kGlu ? glu_act<false>(g1, u1, act, limit) : g1);
-      }
-    }
-    return;
-  }
   for (int n = blockIdx.y * kRows + wi; n < n_end; n += 4) {
     const T* wg = We + (size_t)n * K;
     const T* wu = We + (size_t)(N + n) * K;
@@ -675,6 +845,30 @@ __global__ void __launch_bounds__(128) moe_gemv_kernel(const T* __restrict__ A, 
     if (kGlu) u = warp_sum(u);
     if (lane == 0) out[(size_t)p * ld_out + n] = from_f32<TO>(kGlu ? glu_act<false>(g, u, act, limit) : g);
   }
+}
+
+// One of the two products for a step of few rows. With the activation W [E, 2 N, K], else [E, N, K].
+template <typename T, typename TO, bool kGlu>
+int launch_few(const T* A, long long lda, int a_div, const T* W, TO* out, long long ld_out, const int* ids, int pairs, int E, int N, int K,
+               float limit, int act, cudaStream_t s) {
+  constexpr int kVec = 16 / (int)sizeof(T);
+  const long long stride = (long long)(kGlu ? 2 : 1) * N * K;
+  if (K % kVec != 0 || (uintptr_t)W % 16 != 0) {
+    oi_launch(moe_gemv_kernel<T, TO, kGlu>, dim3(pairs, (N + 15) / 16), 128, (size_t)K * 4, s, A, lda, a_div, W, stride, out, ld_out, ids, E, N, K,
+              limit, act);
+    OI_CHECK_LAUNCH();
+    return OI_OK;
+  }
+  const int fits = kFewInputs / (K * (int)sizeof(T)), at_once = fits < 1 ? 1 : (fits < 4 ? fits : 4);
+  const size_t smem = kFewRing + (size_t)at_once * K * sizeof(T);
+  auto kernel = moe_few_rows_kernel<T, TO, kGlu>;
+  static const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewRing + 48 * 1024);
+  OI_CHECK_CUDA(allowed);
+  const bool x_vec = (uintptr_t)A % 16 == 0 && lda % kVec == 0;
+  oi_launch(kernel, 148 * kFewBlocks, kFewThreads, smem, s, A, lda, a_div, W, stride, out, ld_out, ids, pairs, E, N, K, limit, act, at_once,
+            x_vec ? 1 : 0);
+  OI_CHECK_LAUNCH();
+  return OI_OK;
 }
 
 // add (or null): a float32 term per output number that every row gets beside its experts' sum (an expert all rows share);
@@ -753,7 +947,7 @@ OI_API int oi_moe_tile_rows(int pairs, int experts) {
 
 // Steps of at most this many (row, choice) pairs take the row-by-row products and need no grouping.
 // (None in batch-invariant mode, where a row's sums must be formed the same way whatever else is in the step.)
-OI_API int oi_moe_small(int pairs, int experts) { return !oi_option(OI_OPT_BATCH_INVARIANT) && pairs <= 2 * experts && pairs <= 64; }
+OI_API int oi_moe_small(int pairs, int experts) { return !oi_option(OI_OPT_BATCH_INVARIANT) && pairs <= 2 * experts && pairs <= kFewPairs; }
 
 // x [rows, K] (row stride ldx) in `dtype`; router weights [E, K]; ids, wts [rows, top]; sorted [rows * top];
 // tile_info [3 * max_tiles + 1] with max_tiles = oi_moe_max_tiles(rows * top, E).
@@ -850,33 +1044,18 @@ OI_API int oi_moe_experts(const void* x, int dtype, long long ldx, const void* w
   if (rows == 0) return OI_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const int pairs = rows * top, max_tiles = oi_moe_max_tiles(pairs, E);
-  const bool tma = dtype == OI_BF16 && W % 8 == 0 && F % 8 == 0 && ldx % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)act % 16 == 0 &&
-                   (uintptr_t)w_gate_up % 16 == 0 && (uintptr_t)w_down % 16 == 0;
-  if (oi_moe_small(pairs, E) && tma && glu != OI_ACT_NONE) {
-    int rc = oi_moe_stream(act, F, x, ldx, rows, top, w_gate_up, E, F, W, glu, limit, ids, pairs, stream);
-    if (rc != OI_OK) return rc;
-    rc = oi_moe_stream(y, W, act, F, pairs, 1, w_down, E, W, F, OI_ACT_NONE, 0.f, ids, pairs, stream);
-    if (rc != OI_OK) return rc;
-    return launch_combine(out, y, wts, top, W, rows, add, ids, E, x, dtype, ldx, s);
-  }
   if (oi_moe_small(pairs, E) && (size_t)(W > F ? W : F) * sizeof(float) <= 48 * 1024) {
-    const dim3 v1(pairs, (F + 15) / 16), v2(pairs, (W + 15) / 16);
+    int rc = OI_OK;
     if (dtype == OI_F32) {
-      oi_launch(moe_gemv_kernel<float, float, true>, v1, 128, (size_t)W * 4, s, (const float*)x, ldx, top, (const float*)w_gate_up,
-                (long long)2 * F * W, (float*)act, (long long)F, ids, E, F, W, limit, glu);
-      OI_CHECK_LAUNCH();
-      oi_launch(moe_gemv_kernel<float, float, false>, v2, 128, (size_t)F * 4, s, (const float*)act, (long long)F, 0, (const float*)w_down,
-                (long long)W * F, y, (long long)W, ids, E, W, F, 0.f, 0);
+      rc = launch_few<float, float, true>((const float*)x, ldx, top, (const float*)w_gate_up, (float*)act, F, ids, pairs, E, F, W, limit, glu, s);
+      if (rc == OI_OK) rc = launch_few<float, float, false>((const float*)act, F, 0, (const float*)w_down, y, W, ids, pairs, E, W, F, 0.f, 0, s);
     } else if (dtype == OI_BF16) {
-      oi_launch(moe_gemv_kernel<bf16, bf16, true>, v1, 128, (size_t)W * 4, s, (const bf16*)x, ldx, top, (const bf16*)w_gate_up,
-                (long long)2 * F * W, (bf16*)act, (long long)F, ids, E, F, W, limit, glu);
-      OI_CHECK_LAUNCH();
-      oi_launch(moe_gemv_kernel<bf16, float, false>, v2, 128, (size_t)F * 4, s, (const bf16*)act, (long long)F, 0, (const bf16*)w_down,
-                (long long)W * F, y, (long long)W, ids, E, W, F, 0.f, 0);
+      rc = launch_few<bf16, bf16, true>((const bf16*)x, ldx, top, (const bf16*)w_gate_up, (bf16*)act, F, ids, pairs, E, F, W, limit, glu, s);
+      if (rc == OI_OK) rc = launch_few<bf16, float, false>((const bf16*)act, F, 0, (const bf16*)w_down, y, W, ids, pairs, E, W, F, 0.f, 0, s);
     } else {
       OI_REQUIRE(false, "moe_experts: unknown dtype code %d", dtype);
     }
-    OI_CHECK_LAUNCH();
+    if (rc != OI_OK) return rc;
     return launch_combine(out, y, wts, top, W, rows, add, ids, E, x, dtype, ldx, s);
   }
   const int tile_rows = oi_moe_tile_rows(pairs, E), subs = tile_rows / kTileM;
@@ -893,7 +1072,7 @@ OI_API int oi_moe_experts(const void* x, int dtype, long long ldx, const void* w
     // tensor cores when every row of the operands starts on a 16-byte boundary
     const bool tc1 = W % 8 == 0 && ldx % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w_gate_up % 16 == 0;
     const bool tc2 = F % 8 == 0 && (uintptr_t)act % 16 == 0 && (uintptr_t)w_down % 16 == 0;
-    if (tma && tile_rows == kPairM && (uintptr_t)y % 16 == 0 && glu != OI_ACT_NONE) {
+    if (tc1 && tc2 && tile_rows == kPairM && (uintptr_t)y % 16 == 0 && glu != OI_ACT_NONE) {
       // the sorted rows lie where y will be: the second product writes it, the first reads it
       const size_t pieces = (size_t)pairs * (W / 8);
       const int blocks = (int)((pieces + 255) / 256 > 148 * 8 ? 148 * 8 : (pieces + 255) / 256);

@@ -293,10 +293,6 @@ OI_API int oi_gemm_tcgen05(void* C, int c_dtype, long long ldc, const void* A, l
        ldw, int M, int N, int K, int tile_n, int act, void* stream);
 OI_API int oi_gemm_tcgen05_pair(void* C, int c_dtype, long long ldc, const void* A, long long lda, const void* W, long
        long ldw, int M, int N, int K, int act, void* stream);
-// moe_stream.cu
-OI_API int oi_moe_stream(void* out, long long ld_out, const void* x, long long ldx, int rows, int top, const void* w, int E, int N, int K,
-                         int act, float limit, const int* ids, int pairs, void* stream);
-OI_API int oi_moe_stream_status(int* status);
 // the grouped products of routed experts; `tiles`: [3 * max_tiles + 1] int32 as moe.cu's grouping leaves it
 OI_API int oi_gemm_tcgen05_grouped(void* C, long long ldc, const void* A, long long rows, const void* W, int experts, int N, int K,
                                    int act, float limit, const int* tiles, int max_tiles, const int* sorted, int scatter, void* stream);

@@ -79,7 +79,6 @@ _SIGNATURES = {
     "oi_dyt_step": [P, P, P, P, P, I, P, P, P, I, P, I, P, I, I, P],
     "oi_rope_norm_store": [P, I, L, I, I, I, I, I, P, I, L, P, P, I, I, I, F, P, P, P, P, L, I, I, P],
     "oi_moe_small": [I, I],
-    "oi_moe_stream_status": [ctypes.POINTER(c_int)],
     "oi_joint_norm_rope_store": [P, I, L, I, I, I, I, I, I, I, P, P, F, P, P, I, I, P, P, P, P, L, I, P],
     "oi_sigmoid_attention": [P, L, P, L, P, L, I, P, P, L, I, P, I, P, P, I, I, I, I, F, P, P, P],
     "oi_slice_sum_gate": [P, P, P, P, I, L, P, L, I, I, P],

@@ -5,8 +5,6 @@ the current stream. None of them has another implementation to fall back to.
 """
 from __future__ import annotations
 
-import ctypes
-
 from typing import NamedTuple, Optional
 
 import torch
@@ -749,13 +747,6 @@ def moe_experts(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, 
                                           W, F2 // 2, E, top, float(limit), glu_code(act), ids.data_ptr(), order.data_ptr(), tiles.data_ptr(),
                                           wts.data_ptr(), hidden.data_ptr(), y.data_ptr(), out.data_ptr(), _ptr(add), _stream()), "moe_experts")
     return out
-
-
-def moe_stream_status() -> int:
-    """0, or which bounded wait of the experts' weight stream ran out since the last call (synchronises)."""
-    v = ctypes.c_int(0)
-    _lib.check(_lib.load().oi_moe_stream_status(ctypes.byref(v)), "moe_stream_status")
-    return v.value
 
 
 # ---------------------------------------------------------------------------

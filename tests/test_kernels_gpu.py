@@ -1271,8 +1271,8 @@ def _experts_reference(x, gate_up, down, ids, wts):
     (40, 200, 72, 3, 2), (300, 264, 136, 5, 2), (600, 512, 384, 2, 1), (35, 64, 8, 40, 2), (1300, 72, 264, 4, 3)])   # tiles of 256 places
 @pytest.mark.parametrize("shape", ["spread", "one"])
 def test_routed_experts_bf16_sizes(rows, W, F, E, top, shape):
-    """Edges of the tcgen05 tiles (places, columns, columns of the last 64 along K) and of the weight stream of few rows (16, 32 and 64
-    rows of the second product, K slices), experts that nobody or that everybody chose, more experts than pairs."""
+    """Edges of the tcgen05 tiles (places, columns, columns of the last 64 along K) and of steps of few rows (runs of output rows,
+    remainders along K), experts that nobody or that everybody chose, more experts than pairs."""
     from openinfer_b200.kernels import gemm_tcgen05, ops
     g = torch.Generator().manual_seed(rows + W)
     x = torch.randn(rows, W, generator=g).to(torch.bfloat16).to(DEV)
@@ -1283,7 +1283,61 @@ def test_routed_experts_bf16_sizes(rows, W, F, E, top, shape):
     out = ops.moe_experts(x, gate_up, down, routing, 0.0, act="silu").double()
     ref, bound = _experts_reference(x, gate_up, down, routing[0], routing[1])
     assert ((out - ref).abs() <= bound).all()
-    assert ops.moe_stream_status() == 0 and gemm_tcgen05.status() == 0
+    assert gemm_tcgen05.status() == 0
+
+
+@pytest.mark.parametrize("rows,W,F,E", [(1, 264, 8, 3), (5, 264, 264, 7), (9, 40, 1536, 5), (16, 2048, 2056, 9), (33, 72, 4096, 40), (64, 24, 520, 32)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_experts_of_few_rows_add_in_float32(dtype, rows, W, F, E):
+    """Steps of few rows (up to 64 choices, two an expert on average): every sum is a warp's in float32, a lane's products one after the other,
+    the lanes' sums as a tree. Formed here in the same order and compared bit for bit: the rows are one-hot and the gates 32,
+    whose silu is 32, so that an expert's activations are 32 times a column of its up rows, and a row has one expert."""
+    from openinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(rows + F)
+    gate_up = torch.zeros(E, 2 * F, W)
+    gate_up[:, :F] = 32.0
+    gate_up[:, F:] = torch.randn(E, F, W, generator=g)
+    gate_up, down = gate_up.to(dtype), (torch.randn(E, W, F, generator=g) * F ** -0.5).to(dtype)
+    hot = torch.randint(0, W, (rows,), generator=g)
+    x = torch.nn.functional.one_hot(hot, W).to(dtype)
+    # the first expert has a third of the rows (more than share a pass), another one none
+    chosen = torch.where(torch.arange(rows) % 3 == 0, 0, torch.randint(0, E - 1, (rows,), generator=g))
+    routing = ops.moe_route_table(torch.arange(rows, dtype=torch.int32, device=DEV), chosen.to(torch.int32).view(-1, 1).to(DEV), E)
+    out = ops.moe_experts(x.to(DEV), gate_up.to(DEV), down.to(DEV), routing, 0.0, act="silu").cpu()
+    vec = 8 if dtype == torch.bfloat16 else 4
+    acts = (gate_up[chosen, F:].gather(2, hot.view(-1, 1, 1).expand(rows, F, 1))[:, :, 0].float() * 32.0).to(dtype)
+    steps = -(-F // (32 * vec))
+    pad = steps * 32 * vec - F                                 # (products of zero leave a sum as it is)
+    split = lambda t: torch.nn.functional.pad(t.double(), (0, pad)).view(*t.shape[:-1], steps, 32, vec)      # noqa: E731
+    products = split(down[chosen]) * split(acts).unsqueeze(1)  # exact in float64
+    lanes = torch.zeros(rows, W, 32)
+    for s in range(steps):
+        for e in range(vec):
+            lanes = (lanes.double() + products[:, :, s, :, e]).float()      # a fused multiply-add: one rounding (bfloat16: of an exact product)
+    while lanes.shape[-1] > 1:
+        half = lanes.shape[-1] // 2
+        lanes = lanes[..., :half] + lanes[..., half:]
+    assert torch.equal(out, lanes[..., 0])
+
+
+@pytest.mark.parametrize("rows,E,top", [(1, 4, 2), (7, 16, 2), (20, 40, 3), (40, 3, 2), (300, 5, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_experts_named_twice_by_a_table(dtype, rows, E, top):
+    """A table's row may name an expert twice, or name experts that do not exist (taken as the first or the last one): every entry counts,
+    in steps of few rows as in large ones."""
+    from openinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(rows + E)
+    W, F = 72, 40
+    x = torch.randn(rows, W, generator=g).to(dtype).to(DEV)
+    gate_up = (torch.randn(E, 2 * F, W, generator=g) * W ** -0.5).to(dtype).to(DEV)
+    down = (torch.randn(E, W, F, generator=g) * F ** -0.5).to(dtype).to(DEV)
+    table = torch.randint(0, E, (rows, 1), generator=g).expand(rows, top).clone()
+    table[1::3, 0], table[1::3, 1], table[2::3, 0] = E + 5, E - 1, -1
+    routing = ops.moe_route_table(torch.arange(rows, dtype=torch.int32, device=DEV), table.to(torch.int32).to(DEV), E)
+    assert torch.equal(routing[0].view(rows, top).cpu().long(), table.clamp(0, E - 1))
+    out = ops.moe_experts(x, gate_up, down, routing, 0.0, act="silu").double()
+    ref, bound = _experts_reference(x, gate_up, down, routing[0].view(rows, top), routing[1].view(rows, top))
+    assert ((out - ref).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("E,scoring,groups,keep", [(16, "softmax_top", 1, 1), (20, "sigmoid_groups", 4, 2), (40, "softmax_groups", 5, 3)])
