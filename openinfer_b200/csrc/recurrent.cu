@@ -294,8 +294,9 @@ __device__ __forceinline__ float lanes_sum(float v) {
 // Block (request, head, slice of 2 kThreads / kLanes value columns): the request's rows of the step in order, up to four at a
 // time, the slice of C in registers (the D numbers of two columns spread over kLanes lanes, R of each a lane), the rows' records
 // staged in shared memory a chunk at a time. Two columns share what is read of a row, and the sums over the lanes of four rows
-// are formed by halving. Bound by issue slots (0.75 instructions a clock of a scheduler with one warp). Requests of up to 1,500
-// rows, 8 heads: matrix memory 1,090 -> 766 us with 128 keys and 256 values; linear attention, up to 2,000 rows, 600 -> 410 us.
+// are formed by halving. Bound by issue slots (0.75 instructions a clock of a scheduler with one warp). Four requests of up to
+// 1,500 rows, 8 heads, with the records: matrix memory 1,131 -> 820 us with 128 keys and 256 values; linear attention, up to 2,000
+// rows, 642 -> 468 us. (A lane's read-out in two sums instead of four takes 2 to 3 % less, and loses precision.)
 // Which key channel register i of lane j holds, and a row's D numbers into a thread's R registers. kVec4 (D a multiple of
 // four): a lane holds runs of four neighbours, d = 4 (j + (i / 4) kLanes) + i % 4, and reads them 16 bytes at a time;
 // otherwise d = j + i kLanes.
@@ -399,22 +400,22 @@ __global__ void __launch_bounds__(kThreads) recurrent_scan_kernel(ScanArgs a, in
 #pragma unroll
       for (int e = 0; e < kE; ++e) {
         const float pv = kGates ? put * vals[u * kCols + kE * pair + e] : vals[u * kCols + kE * pair + e];
-        float p[2] = {0.f, 0.f};
+        float p[4] = {0.f, 0.f, 0.f, 0.f};       // four partial sums a lane: short chains of roundings
 #pragma unroll
         for (int i = 0; i < R; ++i) {
           C[e][i] = fmaf(keep, C[e][i], k[i] * pv);
-          p[i & 1] += C[e][i] * q[i];
+          p[i & 3] += C[e][i] * q[i];
         }
-        num[e * 4 + u] = p[0] + p[1];
+        num[e * 4 + u] = (p[0] + p[1]) + (p[2] + p[3]);
       }
       if (kGates) {
-        float p[2] = {0.f, 0.f};
+        float p[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int i = 0; i < R; ++i) {
           nn[i] = fmaf(keep, nn[i], put * k[i]);
-          p[i & 1] += nn[i] * q[i];
+          p[i & 3] += nn[i] * q[i];
         }
-        den[u] = p[0] + p[1];
+        den[u] = (p[0] + p[1]) + (p[2] + p[3]);
       }
     }
 #pragma unroll
@@ -484,8 +485,9 @@ __global__ void __launch_bounds__(kThreads) recurrent_scan_kernel(ScanArgs a, in
 // time (see delta_channel_prepare_kernel). kLanes lanes hold kE = 2 columns of the state, R numbers of each a lane, so that what a
 // run brings is read from shared memory once for both; its sums over the lanes (two columns, four rows, key or query) are
 // formed by halving, every exchange leaving a lane half as many. Bound by shared memory's and the shuffles' pipe: with a
-// column a lane group and two rows at a time (eight trees of shuffles and 24 16-byte reads a pair and column group) requests of
-// up to 1,500 rows, 8 heads of 128 keys and values, took 750 us, and this 382 us (440 us with chunks of 8 rows, 608 us with 8 lanes).
+// column a lane group and two rows at a time (eight trees of shuffles and 24 16-byte reads a pair and column group) four requests
+// of up to 1,500 rows, 8 heads of 128 keys and values, took 788 us with the records, and this 435 us (with one chain of sums a
+// lane instead of four 427 us).
 template <int kLanes, int R, bool kVec4>
 __global__ void __launch_bounds__(kThreads) delta_channel_scan_kernel(ScanArgs a, int chunk) {
   extern __shared__ __align__(16) float stage[];      // two buffers of [chunk / 4] runs, then [chunk][cols] values
@@ -547,16 +549,16 @@ __global__ void __launch_bounds__(kThreads) delta_channel_scan_kernel(ScanArgs a
       }
 #pragma unroll
       for (int e = 0; e < kE; ++e) {
-        float pk = 0.f, pq = 0.f;
+        float pk[4] = {0.f, 0.f, 0.f, 0.f}, pq[4] = {0.f, 0.f, 0.f, 0.f};      // four partial sums a lane, as above
         if (live) {
 #pragma unroll
           for (int i = 0; i < R; ++i) {
-            pk += C[e][i] * k[i];
-            pq += C[e][i] * q[i];
+            pk[i & 3] += C[e][i] * k[i];
+            pq[i & 3] += C[e][i] * q[i];
           }
         }
-        v[(e * 4 + u) * 2] = pk;
-        v[(e * 4 + u) * 2 + 1] = pq;
+        v[(e * 4 + u) * 2] = (pk[0] + pk[1]) + (pk[2] + pk[3]);
+        v[(e * 4 + u) * 2 + 1] = (pq[0] + pq[1]) + (pq[2] + pq[3]);
       }
     }
     float4 s0[4], s1;         // beta, k_0 . k, k_1 . k, k_2 . k of every row; k_0 . q .. k_3 . q of this lane's

@@ -1423,6 +1423,49 @@ def test_recurrent_scan_runs_of_rows(mode, D, V):
                 assert (got[D * V: D * V + D] - n).abs().max() < 3e-5 * (1 + n.abs().max()) and abs(got[-1] - m) < 3e-5 * (1 + abs(m))
 
 
+SCAN_MODES = ["matrix_memory", "gated_delta", "linear_decay"]
+
+
+@pytest.mark.parametrize("mode", SCAN_MODES)
+@pytest.mark.parametrize("rows", [1, 4, 5])
+@pytest.mark.parametrize("requests", [1, 600])
+def test_recurrent_read_outs_add_in_four_sums(mode, rows, requests):
+    """A lane adds its channels of a read-out in four sums, so that what one large term swallows does not add up. The rows leave the state
+    as it is. Column 0 holds 2^25 and, in channels of the same lane that three other sums, or one, or none would take, three numbers of
+    less than half a unit in the last place of that term's product; column 1 the large one alone. Added one by one to the large term
+    they vanish (1.3 units); of four sums only the one that shares its sum is lost."""
+    from types import SimpleNamespace
+
+    from openinfer_b200.kernels import ops
+    D, V, T = 128, 2, rows * requests
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ctx = SimpleNamespace(cu_seqlens=torch.arange(0, T + 1, rows, **i32), token_req=torch.arange(requests, **i32).repeat_interleave(rows),
+                          state_slots=torch.arange(requests, **i32), state_phase=torch.zeros(requests, **i32), num_requests=requests)
+    delta, memory = mode == "gated_delta", mode == "matrix_memory"
+    qkv = torch.zeros(T, 2 * D + V, device=DEV)
+    at = [0, 2, 64, 66]                            # with 8 and with 16 lanes four channels of lane 0: sums 0, 2, 0 and 2 of four
+    qkv[:, at] = 1.0 if delta or memory else 32.0  # silu(32) = 32
+    small = 0.4375 * (2.0 if delta else 4.0)       # of a unit; the unit query of four ones, twice that as q_scale: 1 - 2^-23
+    old = torch.zeros(V, D)
+    old[:, 0] = 2.0 ** 25
+    old[0, at[1:]] = small
+    state = torch.zeros(requests, 2, 1, D * V + (D + 1 if memory else 0), device=DEV)
+    state[:, 0, 0, : D * V] = old.flatten().to(DEV)
+    if memory:                                     # denominator |n . q| = 2^30 (1e-6 more is the same number), and the gates keep everything
+        state[:, 0, 0, D * V + 1], qkv[:, 1] = 2.0 ** 30, 1.0
+    gates = torch.full((T, 2), -200.0, device=DEV)             # delta: beta 0
+    if memory:
+        gates[:, 1] = 200.0
+    out = torch.empty(T, V, device=DEV)
+    code = ops.SCAN_GATED_DELTA if delta else ops.SCAN_MATRIX_MEMORY if memory else ops.SCAN_LINEAR_DECAY
+    ops.recurrent_scan(code, out, qkv, (0, D, 2 * D), gates, (0, 1), state, ctx, 1, 1, D, V,
+                       p0=torch.zeros(D if delta else 1, device=DEV) + (0.0 if delta or memory else 1.0), p1=torch.zeros(1, device=DEV),
+                       decay=torch.full((T, D), -200.0, device=DEV) if delta else None, cap=15.0, q_scale=2.0 if delta else 1.0)
+    out = out.double().cpu() * (2.0 ** 30 if memory else 1.0) / (1.0 if delta or memory else 32.0)
+    unit = 2.0 if delta else 4.0
+    assert ((out[:, 0] - out[:, 1]) - 3 * small).abs().max() <= unit
+
+
 # ------------------------------------------------------------------------------------------------ one block a row, its row in registers
 @pytest.mark.parametrize("hidden", [4, 36, 2048, 2052, 4096, 4100, 8192, 8196, 101])
 @pytest.mark.parametrize("center", [False, True])
