@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "oi_api.h"
 
 namespace {
 
@@ -924,9 +925,14 @@ OI_API int oi_recurrent_scan(int mode, const float* qkv, long long ld_qkv, int q
     OI_CHECK_LAUNCH();
     return OI_OK;
   }
-  // Lanes a column: with eight an SM's schedulers issue least, with sixteen a run's chain is shorter and there are twice the
-  // blocks, which counts while the blocks of eight lanes would leave SMs with a few warps.
-  const bool few = (long long)requests * H * ((V + 31) / 32) < 4 * 148;
+  // Lanes a column where either form takes the head: with eight an SM's schedulers issue least, with sixteen a run's chain is
+  // shorter and there are twice the blocks, which counts while the blocks of eight lanes would be fewer than three for two SMs.
+  // us with 8 / 16 lanes, 8 heads, requests of up to 1,500 rows (the records included): delta rule (128 values) 1 request 425 / 316,
+  // 4 458 / 435, 6 (192 blocks of eight lanes) 625 / 572, 8 (256) 645 / 786, 16 1,095 / 1,255; matrix memory (256 values) 1 request
+  // 453 / 377, 2 471 / 493, 3 (192) 650 / 640, 4 (256) 660 / 821, 16 1,927 / 2,351. The two add a row's products in another order, so
+  // in batch-invariant mode it is eight whatever the step; the linear decay takes sixteen whatever the step (up to 2,000 rows:
+  // 1 request 426 / 349, 4 458 / 468, 8 657 / 753).
+  const bool few = !oi_option(OI_OPT_BATCH_INVARIANT) && (long long)requests * H * ((V + 31) / 32) < 222;
   if (mode == kGatedDelta) {
     const int rows = D <= 128 ? 16 : 4;                         // per buffer: two buffers of at most 30 KB
 #define OI_DELTA_CHANNEL(LANES, REGS)                                                                                       \
@@ -961,17 +967,17 @@ OI_API int oi_recurrent_scan(int mode, const float* qkv, long long ld_qkv, int q
     if (smem > 48 * 1024) OI_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
     oi_launch(kernel, grid, kThreads, smem, s, a, chunk);                                                               \
   } while (0)
-#define OI_SCAN(MODE)                                   \
-  do {                                                  \
-    if (D <= 32) OI_SCAN_AS(MODE, 8, 4);                \
-    else if (D <= 64) OI_SCAN_AS(MODE, 16, 4);          \
-    else if (D <= 128 && few) OI_SCAN_AS(MODE, 16, 8);  \
-    else if (D <= 128) OI_SCAN_AS(MODE, 8, 16);         \
-    else if (D <= 256) OI_SCAN_AS(MODE, 32, 8);         \
-    else OI_SCAN_AS(MODE, 32, 16);                      \
+#define OI_SCAN(MODE, UP_TO_128)                 \
+  do {                                           \
+    if (D <= 32) OI_SCAN_AS(MODE, 8, 4);         \
+    else if (D <= 64) OI_SCAN_AS(MODE, 16, 4);   \
+    else if (D <= 128) UP_TO_128;                \
+    else if (D <= 256) OI_SCAN_AS(MODE, 32, 8);  \
+    else OI_SCAN_AS(MODE, 32, 16);               \
   } while (0)
-  if (mode == kMatrixMemory) OI_SCAN(kMatrixMemory);
-  else OI_SCAN(kLinearDecay);
+  if (mode == kLinearDecay) OI_SCAN(kLinearDecay, OI_SCAN_AS(kLinearDecay, 16, 8));
+  else if (few) OI_SCAN(kMatrixMemory, OI_SCAN_AS(kMatrixMemory, 16, 8));
+  else OI_SCAN(kMatrixMemory, OI_SCAN_AS(kMatrixMemory, 8, 16));
 #undef OI_SCAN
 #undef OI_SCAN_AS
   OI_CHECK_LAUNCH();

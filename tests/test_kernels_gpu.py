@@ -1466,6 +1466,103 @@ def test_recurrent_read_outs_add_in_four_sums(mode, rows, requests):
     assert ((out[:, 0] - out[:, 1]) - 3 * small).abs().max() <= unit
 
 
+def _scan_inputs(mode, lens, H, G, D, V, seed):
+    from types import SimpleNamespace
+    g = torch.Generator().manual_seed(seed)
+    T, B = sum(lens), len(lens)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    cu = [sum(lens[:b]) for b in range(B + 1)]
+    ctx = SimpleNamespace(cu_seqlens=torch.tensor(cu, **i32), token_req=torch.tensor([b for b, n in enumerate(lens) for _ in range(n)], **i32),
+                          state_slots=torch.arange(B, **i32), state_phase=torch.tensor([b % 2 for b in range(B)], **i32), num_requests=B)
+    delta, memory = mode == "gated_delta", mode == "matrix_memory"
+    rand = lambda *shape: torch.randn(*shape, generator=g)      # noqa: E731
+    t = SimpleNamespace(qkv=rand(T, 2 * G * D + H * V), gates=rand(T, 2 * H), state=rand(B, 2, H, D * V + (D + 1 if memory else 0)) * 0.3,
+                        decay=rand(T, H * D), p0=rand(H * D if delta else H) * 0.3, p1=rand(H) * 0.3)
+    if memory:
+        t.state[..., -1].abs_()
+    if not (delta or memory):
+        t.p0 = t.p0.sigmoid()
+    return ctx, cu, t
+
+
+def _run_scan(mode, ctx, t, H, G, D, V):
+    """(out, state behind the step); the inputs stay as they are."""
+    from openinfer_b200.kernels import ops
+    qkv, gates, state, decay, p0, p1 = (v.to(DEV, copy=True) for v in (t.qkv, t.gates, t.state, t.decay, t.p0, t.p1))
+    out = torch.empty(qkv.shape[0], H * V, device=DEV)
+    code = {"gated_delta": ops.SCAN_GATED_DELTA, "matrix_memory": ops.SCAN_MATRIX_MEMORY, "linear_decay": ops.SCAN_LINEAR_DECAY}[mode]
+    ops.recurrent_scan(code, out, qkv, (0, G * D, 2 * G * D), gates, (0, H), state, ctx, H, G, D, V, p0=p0, p1=p1,
+                       decay=decay if mode == "gated_delta" else None, cap=15.0, q_scale=D ** -0.5)
+    return out.cpu(), state.cpu()
+
+
+@pytest.mark.parametrize("mode", SCAN_MODES)
+@pytest.mark.parametrize("D", [100, 128])
+def test_recurrent_scan_of_many_blocks(mode, D):
+    """Enough requests, heads and columns (40 x 4 x 128: 640 blocks of 32) for the split that large steps take of 65 to 128 key channels,
+    with whole runs of four rows, parts of one, and more than a chunk of sixteen; row by row in float64."""
+    lens, H, G, V = [1, 4, 3, 6, 2, 5, 8, 1, 4, 19] * 4, 4, 2, 128
+    ctx, cu, t = _scan_inputs(mode, lens, H, G, D, V, D)
+    out, after = _run_scan(mode, ctx, t, H, G, D, V)
+    delta, memory = mode == "gated_delta", mode == "matrix_memory"
+    x, g, dc, p0, p1 = (v.double() for v in (t.qkv, t.gates, t.decay, t.p0, t.p1))
+    if not (delta or memory):
+        x = torch.nn.functional.silu(x)
+    q, k = (x[:, at: at + G * D].view(-1, G, D).repeat_interleave(H // G, dim=1) for at in (0, G * D))
+    v = x[:, 2 * G * D:].view(-1, H, V)
+    dot = lambda C, u: torch.einsum("hvd,hd->hv", C, u)      # noqa: E731
+    for b in range(len(lens)):
+        old = t.state[b, b % 2].double()
+        C, n, m = old[:, : D * V].view(H, V, D), old[:, D * V: D * V + D], old[:, -1]
+        for r in range(cu[b], cu[b + 1]):
+            kt, qt, low = k[r], q[r] * D ** -0.5, 1.0
+            if delta:
+                kt, qt = kt / (kt.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt(), qt / (q[r].pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()
+                C = C * torch.exp(-p1.exp()[:, None] * torch.nn.functional.softplus(dc[r].view(H, D) + p0.view(H, D)))[:, None]
+                C = C + (torch.sigmoid(g[r, :H])[:, None] * (v[r] - dot(C, kt)))[:, :, None] * kt[:, None]
+                o = dot(C, qt)
+            elif not memory:
+                C = p0[:, None, None] * C + v[r][:, :, None] * kt[:, None]
+                o = dot(C, qt)
+            else:
+                i, f = 15 * torch.tanh((g[r, :H] + p0) / 15), torch.nn.functional.logsigmoid(15 * torch.tanh((g[r, H:] + p1) / 15))
+                new = torch.maximum(f + m, i)
+                keep, put, m = torch.exp(f + m - new), torch.exp(i - new), new
+                C, n = keep[:, None, None] * C + put[:, None, None] * v[r][:, :, None] * kt[:, None], keep[:, None] * n + put[:, None] * kt
+                low = torch.maximum((n * qt).sum(-1).abs(), torch.exp(-m)).clamp(max=1.0)[:, None]
+                o = dot(C, qt) / (torch.maximum((n * qt).sum(-1).abs(), torch.exp(-m)) + 1e-6)[:, None]
+            # as above: 19 steps of sums of up to 128 float32 products, and a denominator that may be small
+            assert ((out[r].double().view(H, V) - o).abs() < 3e-5 * (1 + C.abs().max() + o.abs().max()) / low).all()
+        got = after[b, 1 - b % 2].double()
+        assert (got[:, : D * V].view(H, V, D) - C).abs().max() < 3e-5 * (1 + C.abs().max())
+        if memory:
+            assert (got[:, D * V: D * V + D] - n).abs().max() < 3e-5 * (1 + n.abs().max()) and (got[:, -1] - m).abs().max() < 3e-5 * (1 + m.abs().max())
+
+
+@pytest.mark.parametrize("mode", SCAN_MODES)
+@pytest.mark.parametrize("D", [64, 100, 128, 132])
+def test_recurrent_scan_in_batch_invariant_mode(mode, D):
+    """In batch-invariant mode a request's read-outs and state are the same bit for bit alone and among others, however many."""
+    from types import SimpleNamespace
+
+    from openinfer_b200.kernels import policy
+    H, G, V, lens = 8, 8, 128, [9, 1, 4, 2] * 6
+    ctx, cu, t = _scan_inputs(mode, lens, H, G, D, V, D + 1)
+    policy.set_batch_invariant(True)
+    try:
+        out, after = _run_scan(mode, ctx, t, H, G, D, V)
+        for b in (0, 1, 23):
+            rows = slice(cu[b], cu[b + 1])
+            one = SimpleNamespace(cu_seqlens=torch.tensor([0, lens[b]], dtype=torch.int32, device=DEV),
+                                  token_req=torch.zeros(lens[b], dtype=torch.int32, device=DEV),
+                                  state_slots=torch.zeros(1, dtype=torch.int32, device=DEV), state_phase=ctx.state_phase[b: b + 1], num_requests=1)
+            alone = SimpleNamespace(qkv=t.qkv[rows], gates=t.gates[rows], state=t.state[b: b + 1], decay=t.decay[rows], p0=t.p0, p1=t.p1)
+            o, s = _run_scan(mode, one, alone, H, G, D, V)
+            assert torch.equal(o, out[rows]) and torch.equal(s[0], after[b])
+    finally:
+        policy.set_batch_invariant(False)
+
+
 # ------------------------------------------------------------------------------------------------ one block a row, its row in registers
 @pytest.mark.parametrize("hidden", [4, 36, 2048, 2052, 4096, 4100, 8192, 8196, 101])
 @pytest.mark.parametrize("center", [False, True])
