@@ -269,6 +269,32 @@ __global__ void __launch_bounds__(kGroupThreads) moe_group_kernel(const int* __r
   }
 }
 
+// The b-th run of up to kTileM places of the list's tiles, however tall those are: expert, first place, rows. False behind the last
+// one. Every warp looks through the list by itself.
+__device__ __forceinline__ bool run_of_places(const int* __restrict__ tile_info, int max_tiles, int b, int& e, int& place0, int& m_rows) {
+  const int lane = threadIdx.x & 31, tiles = min(tile_info[3 * max_tiles], max_tiles);
+  int before = 0;
+  for (int t0 = 0; t0 < tiles; t0 += 32) {
+    const int t = t0 + lane, rows = t < tiles ? tile_info[3 * t + 2] : 0, runs = (rows + kTileM - 1) / kTileM;
+    int upto = before + runs;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, upto - before, o);
+      if (lane >= o) upto += up;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, upto > b);
+    if (hit) {
+      const int from = __ffs(hit) - 1, part = b - __shfl_sync(0xffffffffu, upto - runs, from);
+      e = tile_info[3 * (t0 + from)];
+      place0 = tile_info[3 * (t0 + from) + 1] + part * kTileM;
+      m_rows = min(__shfl_sync(0xffffffffu, rows, from) - part * kTileM, kTileM);
+      return true;
+    }
+    before = __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return false;
+}
+
 // out rows of one tile: C[i, n] = sum_k A[src(i), k] * W_e[n, k] (k ascending), i over the tile's sorted places.
 // kGlu: W_e holds N gate rows and then N up rows; the result is the gated activation `act` of the two sums (glu_act:
 // act(g) * u, or with OI_ACT_SWIGLU_CLAMP g' sigmoid(1.702 g') (u' + 1) with g' = min(g, limit), u' = clamp(u, -limit, limit)). a_div: the source row of place i is sorted[i] / a_div (a_div 0: the place itself).
@@ -279,12 +305,8 @@ __global__ void __launch_bounds__(256) moe_gemm_kernel(const T* __restrict__ A, 
                                                        const int* __restrict__ sorted, const int* __restrict__ tile_info,
                                                        int max_tiles, int N, int K, float limit, int act) {
   pdl_wait();    // no early trigger: waiting blocks of the next kernel would share the SMs with this product
-  const int tile = blockIdx.x;
-  if (tile >= tile_info[3 * max_tiles]) return;
-  // a block takes kTileM rows: of a longer tile, the part that blockIdx.z names
-  const int e = tile_info[3 * tile], place0 = tile_info[3 * tile + 1] + (int)blockIdx.z * kTileM;
-  const int m_rows = min(tile_info[3 * tile + 2] - (int)blockIdx.z * kTileM, kTileM);
-  if (m_rows <= 0) return;
+  int e, place0, m_rows;
+  if (!run_of_places(tile_info, max_tiles, blockIdx.x, e, place0, m_rows)) return;
   const int n0 = blockIdx.y * kTileN;
   __shared__ float As[kTileK][kTileM + 1];
   __shared__ float Wg[kTileK][kTileN + 1];
@@ -396,12 +418,8 @@ __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const bf16* __restric
                                                            int scatter, const int* __restrict__ sorted,
                                                            const int* __restrict__ tile_info, int max_tiles, int N, int K, float limit, int act) {
   pdl_wait();
-  const int tile = blockIdx.x;
-  if (tile >= tile_info[3 * max_tiles]) return;
-  // a block takes kTileM rows: of a longer tile, the part that blockIdx.z names
-  const int e = tile_info[3 * tile], place0 = tile_info[3 * tile + 1] + (int)blockIdx.z * kTileM;
-  const int m_rows = min(tile_info[3 * tile + 2] - (int)blockIdx.z * kTileM, kTileM);
-  if (m_rows <= 0) return;
+  int e, place0, m_rows;
+  if (!run_of_places(tile_info, max_tiles, blockIdx.x, e, place0, m_rows)) return;
   const int n0 = blockIdx.y * kTileN;
   constexpr int kPad = kTileK + 8;
   __shared__ __align__(16) bf16 As[kTileM][kPad];
@@ -1058,10 +1076,10 @@ OI_API int oi_moe_experts(const void* x, int dtype, long long ldx, const void* w
     if (rc != OI_OK) return rc;
     return launch_combine(out, y, wts, top, W, rows, add, ids, E, x, dtype, ldx, s);
   }
-  const int tile_rows = oi_moe_tile_rows(pairs, E), subs = tile_rows / kTileM;
+  const int tile_rows = oi_moe_tile_rows(pairs, E);
   const bool big = tile_rows == kBigM;
-  const dim3 g1(max_tiles, (F + kTileN - 1) / kTileN, subs), g2(max_tiles, (W + kTileN - 1) / kTileN, subs);
-  const dim3 b1(max_tiles, (F + kTileN - 1) / kTileN), b2(max_tiles, (W + kTileN - 1) / kTileN);
+  // a block a run of 32 places, of which there are no more than max_tiles (or, of 128 places, a tile) and 64 output rows
+  const dim3 g1(max_tiles, (F + kTileN - 1) / kTileN), g2(max_tiles, (W + kTileN - 1) / kTileN);
   if (dtype == OI_F32) {
     oi_launch(moe_gemm_kernel<float, float, true>, g1, 256, 0, s, (const float*)x, ldx, top, (const float*)w_gate_up, (long long)2 * F * W,
               (float*)act, (long long)F, 0, sorted, tile_info, max_tiles, F, W, limit, glu);
@@ -1085,7 +1103,7 @@ OI_API int oi_moe_experts(const void* x, int dtype, long long ldx, const void* w
       return launch_combine(out, y, wts, top, W, rows, add, ids, E, x, dtype, ldx, s);
     }
     if (tc1 && big)
-      oi_launch(moe_gemm_mma_big_kernel<bf16, true>, b1, 256, 0, s, (const bf16*)x, ldx, top, (const bf16*)w_gate_up, (long long)2 * F * W,
+      oi_launch(moe_gemm_mma_big_kernel<bf16, true>, g1, 256, 0, s, (const bf16*)x, ldx, top, (const bf16*)w_gate_up, (long long)2 * F * W,
                 (bf16*)act, (long long)F, 0, sorted, tile_info, max_tiles, F, W, limit, glu);
     else if (tc1)
       oi_launch(moe_gemm_mma_kernel<bf16, true>, g1, 256, 0, s, (const bf16*)x, ldx, top, (const bf16*)w_gate_up, (long long)2 * F * W,
@@ -1095,7 +1113,7 @@ OI_API int oi_moe_experts(const void* x, int dtype, long long ldx, const void* w
                 (bf16*)act, (long long)F, 0, sorted, tile_info, max_tiles, F, W, limit, glu);
     OI_CHECK_LAUNCH();
     if (tc2 && big)
-      oi_launch(moe_gemm_mma_big_kernel<float, false>, b2, 256, 0, s, (const bf16*)act, (long long)F, 0, (const bf16*)w_down, (long long)W * F,
+      oi_launch(moe_gemm_mma_big_kernel<float, false>, g2, 256, 0, s, (const bf16*)act, (long long)F, 0, (const bf16*)w_down, (long long)W * F,
                 y, (long long)W, 1, sorted, tile_info, max_tiles, W, F, 0.f, 0);
     else if (tc2)
       oi_launch(moe_gemm_mma_kernel<float, false>, g2, 256, 0, s, (const bf16*)act, (long long)F, 0, (const bf16*)w_down, (long long)W * F,
