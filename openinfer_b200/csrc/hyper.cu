@@ -5,6 +5,7 @@
 // single-stream layers. With S = 1 and no coefficients (a = b = 1, M = 1) this is the plain pre-norm residual on a
 // float32 stream.
 #include "common.cuh"
+#include "oi_api.h"
 
 namespace {
 
@@ -188,8 +189,9 @@ OI_API int oi_hyper_step(float* X, int rows, int S, int W, const float* y, const
   const bool vec = W % 4 == 0 && (uintptr_t)X % 16 == 0 && (y == nullptr || (uintptr_t)y % 16 == 0) && (y2 == nullptr || (uintptr_t)y2 % 16 == 0);
   const int cols = vec ? W / 4 : W;
   // At least S * S threads. Few rows of up to four streams keep every column in a thread's registers: 4 rows of two streams of
-  // 2,048 6.4 -> 4.1 us. Many rows are better off with more blocks on an SM: 4,200 rows 43 us, kept in registers 53 us.
-  const int keep = rows <= 4 * 148 && S <= 4 && vec && cols <= 1024 && (out == nullptr || (uintptr_t)out % 8 == 0) ? (cols <= 512 ? 1 : 2) : 0;
+  // 2,048 6.4 -> 4.1 us. Many rows are better off with more blocks on an SM: 4,200 rows 43 us, kept in registers 53 us. The two
+  // forms add a row's squares in another order, so in batch-invariant mode every step takes the one for many rows.
+  const int keep = rows <= 4 * 148 && !oi_option(OI_OPT_BATCH_INVARIANT) && S <= 4 && vec && cols <= 1024 && (out == nullptr || (uintptr_t)out % 8 == 0) ? (cols <= 512 ? 1 : 2) : 0;
   const int threads = keep ? ((cols + keep - 1) / keep + 31) / 32 * 32 : ((cols >= 1024 || S > 8) ? 256 : (cols >= 256 ? 128 : 64));
   cudaStream_t s = (cudaStream_t)stream;
 #define OI_HYPER_S(TO, VEC, MAXS, KEEP)                                                                                    \

@@ -15,7 +15,16 @@ def luzitar():
             "layers": [{"type": "lightning", "mixer": linear, "mlp": mlp}, {"type": "attention", "mixer": attention, "mlp": mlp}]}
 
 
-MAKERS = {"luzitar": luzitar}
+def pilonex():
+    left = {"heads": 4, "kv_heads": 2, "dim": 64, "vdim": 64, "scale": 0.125, "mask": {"size": 48}, "rot": {"dims": 64, "base": 10000.0}}
+    right = {"heads": 8, "kv_heads": 4, "dim": 128, "vdim": 128, "conv": 4, "decay_rank": 32, "gate_rank": 32}
+    mlp = {"kind": "dense", "ff": 256, "limit": 7.0}
+    return {"architecture": "Pilonex", "vocab": VOCAB, "width": WIDTH, "norm": {"eps": 1e-6}, "streams": 2,
+            "layers": [{"type": "parallel", "mixer": {"left": left, "right": right, "left_scale": 1.0, "right_scale": 1.0}, "mlp": mlp},
+                       {"type": "mlstm", "mixer": {"heads": 8, "dim": 128, "vdim": 128, "gate_cap": 15.0}, "mlp": mlp}]}
+
+
+MAKERS = {"luzitar": luzitar, "pilonex": pilonex}
 
 
 @pytest.mark.parametrize("name", sorted(MAKERS))

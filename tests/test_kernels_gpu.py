@@ -1605,6 +1605,53 @@ def test_hyper_step_widths(S, W, dst):
     assert ((out.cpu().double() - ref).abs() <= ref.abs() * (step + 2.0 ** -18) + slack).all()
 
 
+def _hyper_inputs(rows, S, W):
+    g = torch.Generator().manual_seed(S * W + rows)
+    shapes = dict(X=(rows, S, W), y=(rows, W), mix=(S, S), b_out=(S,), a_in=(S,), norm_w=(W,))
+    return {name: torch.randn(*shape, generator=g) for name, shape in shapes.items()}
+
+
+def _run_hyper(t, rows, dst):
+    from openinfer_b200.kernels import ops
+    t = {name: (v[rows] if name in "Xy" else v).to(DEV, copy=True) for name, v in t.items()}
+    X, out = t.pop("X"), torch.empty(t["y"].shape, dtype=dst, device=DEV)
+    ops.hyper_step(X, eps=1e-5, weight_offset=1.0, out=out, **t)
+    return X.cpu(), out.cpu()
+
+
+@pytest.mark.parametrize("S,W", [(2, 2048), (4, 4096), (1, 36)])
+@pytest.mark.parametrize("dst", [torch.float32, torch.bfloat16])
+def test_hyper_step_of_many_rows(S, W, dst):
+    """From 593 rows on a thread walks its columns twice and keeps none of them."""
+    t = _hyper_inputs(593, S, W)
+    X, out = _run_hyper(t, slice(None), dst)
+    d = {name: v.double() for name, v in t.items()}
+    new = torch.einsum("sr,tsw->trw", d["mix"], d["X"]) + d["b_out"][None, :, None] * d["y"][:, None]
+    u = torch.einsum("s,tsw->tw", d["a_in"], new)
+    ref = u * torch.rsqrt(u.pow(2).mean(-1, keepdim=True) + 1e-5) * (1.0 + d["norm_w"])
+    # as above
+    assert (X.double() - new).abs().max() <= 2.0 ** -17
+    step = 2.0 ** -8 if dst == torch.bfloat16 else 0.0
+    slack = 2.0 ** -14 * (1.0 + d["norm_w"].abs()) / u.pow(2).mean(-1, keepdim=True).sqrt().clamp(max=1.0)
+    assert ((out.double() - ref).abs() <= ref.abs() * (step + 2.0 ** -18) + slack).all()
+
+
+@pytest.mark.parametrize("S,W", [(2, 2048), (3, 1024), (4, 4096), (2, 512)])
+@pytest.mark.parametrize("dst", [torch.float32, torch.bfloat16])
+def test_hyper_step_in_batch_invariant_mode(S, W, dst):
+    """In batch-invariant mode a row is the same bit for bit in a step of 592 rows and in one of 700 (of rows whose squares are added in
+    another order one in ten differs)."""
+    from openinfer_b200.kernels import policy
+    t = _hyper_inputs(700, S, W)
+    policy.set_batch_invariant(True)
+    try:
+        X, out = _run_hyper(t, slice(None), dst)
+        few_X, few = _run_hyper(t, slice(0, 592), dst)
+    finally:
+        policy.set_batch_invariant(False)
+    assert torch.equal(few, out[:592]) and torch.equal(few_X, X[:592])
+
+
 @pytest.mark.parametrize("hidden", [4, 132, 2048, 2056, 6])
 def test_embedding_widened(hidden):
     from openinfer_b200.kernels import ops
