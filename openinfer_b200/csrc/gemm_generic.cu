@@ -317,11 +317,13 @@ int launch_rows(void* C, const void* A, const void* W, int M, int N, int K, long
 template <typename TA, typename TW, typename TC>
 int launch(void* C, const void* A, const void* W, int M, int N, int K, long long lda, long long ldw,
            long long ldc, cudaStream_t s) {
-  // The stream's time grows with the rows (a term of A is read from shared memory for every 8 weight rows), that of a row of
-  // tiles does not up to 64 rows, but few tiles leave SMs idle. us, stream / tiles: N 4096 K 1024 at 32 rows 32 / 33, at
-  // 48 44 / 33; N 6144 K 1024 at 32 44 / 60, at 48 66 / 60; N 6144 K 4096 at 32 211 / 235, at 48 317 / 235; N 4096 K 12288 at
-  // 16 221 / 364, at 32 440 / 364; N 1024 K 3072 at 64 46 / 93; N 1024 K 2048 at 64 32 / 63.
-  const bool stream = M <= 32 || (M <= 64 && N <= 2048);
+  // The stream's time grows with groups of eight rows times N (2.0 ns a column and group at K = 1,024), that of a row of tiles not at
+  // all up to 64 rows and with the waves of tiles beyond one an SM (30 us each at K = 1,024); both with K alike. us, stream /
+  // tiles: N 4096, 3 groups K 1024 24 / 32, K 12288 346 / 353, 4 groups 32 / 32, 442 / 357; N 6144 K 4096 2 groups 112 / 120, 3 162 / 121;
+  // N 12288 K 2048 2 groups 111 / 119, 3 161 / 119; N 24576 K 4096 1 group 214 / 351, 2 421 / 353; N 1024 K 3072 8 groups 47 / 93;
+  // N 2048, 8 groups K 1024 32 / 33, K 2048 54 / 64.
+  const long long groups_of_rows = (M + 7) / 8, waves = (N + 148 * BN - 1) / (148 * BN);
+  const bool stream = M <= 64 && groups_of_rows * N < 15500 * waves;
   if (stream && K <= 32768 && aligned_rows(A, lda, sizeof(TA), 16) && aligned_rows(W, ldw, sizeof(TW), 16)) {
     if (M == 1) return launch_rows<TA, TW, TC, 1>(C, A, W, M, N, K, lda, ldw, ldc, s);
     if (M == 2) return launch_rows<TA, TW, TC, 2>(C, A, W, M, N, K, lda, ldw, ldc, s);

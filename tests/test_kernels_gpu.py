@@ -218,7 +218,7 @@ def test_attention_generic(dtype, nq, nkv, hd, P, window):
 @pytest.mark.parametrize("a_dtype,w_dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
 @pytest.mark.parametrize("M,N,K", [(1, 8, 256), (2, 41, 260), (3, 1000, 1024), (7, 24, 3080), (9, 8, 16), (64, 72, 520), (5, 9500, 264), (8, 16, 12288)])
 def test_gemm_generic_few_rows(a_dtype, w_dtype, M, N, K):
-    """The weight stream (up to 32 rows, narrow products up to 64): remainders of its 8 weight rows, of its runs of 1,024 terms and of its row groups, several
+    """The weight stream (few rows): remainders of its 8 weight rows, of its runs of 1,024 terms and of its row groups, several
     groups of weight rows in a block, K beyond one run of its warps. The sums are those of the tile kernel, bit for bit."""
     from openinfer_b200.kernels import ops
     a = torch.randn(M, K, device=DEV).to(a_dtype)
@@ -231,6 +231,20 @@ def test_gemm_generic_few_rows(a_dtype, w_dtype, M, N, K):
     many = torch.empty(65, N, device=DEV, dtype=torch.float32)
     ops.gemm_generic(many, torch.cat([a, torch.zeros(65 - M, K, device=DEV, dtype=a_dtype)]), w)
     assert torch.equal(many[:M], out)
+
+
+@pytest.mark.parametrize("M,N", [(24, 4096), (25, 4096), (16, 6144), (17, 6144), (64, 1936), (64, 1938), (8, 9480), (16, 15499), (17, 9473)])
+def test_gemm_generic_on_both_sides_of_the_rule(M, N):
+    """Rows times columns up to which the weight stream is taken, and just beyond: the same sums bit for bit as in a large product, and those of float64."""
+    from openinfer_b200.kernels import ops
+    K = 264
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    out, many = torch.empty(M, N, device=DEV), torch.empty(130, N, device=DEV)
+    ops.gemm_generic(out, a, w)
+    ops.gemm_generic(many, torch.cat([a, torch.zeros(130 - M, K, device=DEV)]), w)
+    assert torch.equal(many[:M], out)
+    # as above
+    assert (out.double() - a.double() @ w.double().t()).abs().max() < 2.0 ** -24 * (16 + (K / 256) ** 0.5) * 8 * K ** 0.5
 
 
 @pytest.mark.parametrize("S", [1, 31, 32, 33, 255, 256, 257, 289, 1000])
