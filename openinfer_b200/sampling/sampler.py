@@ -100,7 +100,7 @@ class Sampler:
             idx = dev[5 * k: 6 * k]
             if self._probs is None or self._probs.numel() < k * self.vocab_size:
                 self._probs = torch.empty(k * self.vocab_size, dtype=torch.float32, device=self.device)
-            if logits.stride(1) != 1:
+            if logits.stride(1) != 1 or logits.stride(0) < self.vocab_size:      # (one row for several requests, say)
                 logits = logits.contiguous()
             # the kernel reads the sampled rows where they are and writes their places: greedy rows keep their argmax
             ops.sample(out, logits, self._probs, fl[0], tk, fl[1], fl[2], fl[3], row_idx=None if k == n else idx)

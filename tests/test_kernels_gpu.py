@@ -409,6 +409,19 @@ def test_sample_by_clusters_keeps_what_one_block_keeps(vocab, spread):
         assert out == [got[True][r] if r in (21, 3, 8) else 77 for r in range(rows)]
 
 
+def test_sampler_draws_from_any_layout_of_the_logits():
+    """Rows that all requests sample from may be one row expanded, columns of a wider tensor or a transposed tensor."""
+    from openinfer_b200 import SamplingParams
+    from openinfer_b200.sampling.sampler import Sampler
+    vocab, n = 1000, 5
+    torch.manual_seed(3)
+    sampler = Sampler(vocab, torch.device(DEV))
+    params = [SamplingParams(temperature=0.9, top_k=40, seed=i) for i in range(n)]
+    wide = torch.randn(n, vocab + 7, device=DEV)
+    for logits in (wide[:1, :vocab].expand(n, vocab), wide[:, 3: vocab + 3], wide[:, :vocab].t().contiguous().t()):
+        assert sampler.select(logits, params, list(range(n)), 1) == sampler.select(logits.clone(memory_format=torch.contiguous_format), params, list(range(n)), 1)
+
+
 def test_sample_when_the_estimate_of_the_candidate_list_is_wrong(sample_clusters):
     """The kernel places the cut of its shared-memory list from a histogram of one value in eight (the first of
     every other group of four per thread). 5,000 equal large values at places that are never counted make that
