@@ -552,9 +552,9 @@ __global__ void __launch_bounds__(256) short_conv_vec_kernel(
         for (int e = 0; e < 4; ++e) wt[j][e] = load_as_f32(w, w_dtype, (size_t)(c + e) * taps + keep - j);   // of the input j rows above
       }
   }
-  // What depends on no kernel of the step, before the wait: the requests of the rows and of the taps - 1 rows above them (a
-  // request's rows are consecutive, so a row's place in its portion shows in its neighbours' requests alone), and, where a
-  // thread has one row, the old state that this row needs.
+  // What depends on no kernel, before the wait: the requests of the rows and of the taps - 1 rows above them (a request's rows are
+  // consecutive, so a row's place in its portion shows in its neighbours' requests alone). Where a thread has one row, the old
+  // state that this row needs is asked for first behind it: it may be what the kernel before leaves behind.
   const int t_end = min(tokens, t0 + kRows);
   int reqs[kRows + kTaps - 1];
 #pragma unroll
@@ -569,6 +569,7 @@ __global__ void __launch_bounds__(256) short_conv_vec_kernel(
       if (j <= keep && rel == j - 1 && reqs[i + kTaps - 1 - j] == reqs[i + kTaps - 1]) rel = j;
     return rel;
   };
+  pdl_wait();
   float early[kRows == 1 ? kTaps : 1][4];      // early[j]: the state's row that stands j rows above this one
   if (kRows == 1 && t0 < t_end && c < channels) {
     const int req = reqs[kTaps - 1], rel = place(0);
@@ -579,7 +580,6 @@ __global__ void __launch_bounds__(256) short_conv_vec_kernel(
         if (j <= keep && j > rel) load4(st + (size_t)(keep + rel - j) * channels + c, early[kRows == 1 ? j : 0]);
     }
   }
-  pdl_wait();
   if (c >= channels) return;
   // ring[i]: the input i + 1 rows above the current one
   float ring[kTaps][4];

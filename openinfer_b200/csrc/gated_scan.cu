@@ -188,13 +188,13 @@ __global__ void mingru_step_kernel(TO* out, long long out_stride, const float* z
                                    const int* __restrict__ cu_seqlens, const int* __restrict__ token_req,
                                    const int* __restrict__ state_slots, int channels) {
   pdl_trigger();
-  // the metadata, the biases and the old state depend on no kernel of the step: before the wait
+  // the metadata and the biases depend on no kernel: before the wait. The old state may be what the kernel before leaves behind.
   const int b = blockIdx.x, t = cu_seqlens[b];
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   const bool live = cu_seqlens[b + 1] - t == 1 && c < channels, padding = live && token_req[t] < 0;
   float* st = state + (size_t)state_slots[b] * state_stride + c;
-  float old = 0.f, bz = 0.f, bx = 0.f;
-  if (live && !padding) old = *st, bz = bias[c], bx = bias[channels + c];
+  float bz = 0.f, bx = 0.f;
+  if (live && !padding) bz = bias[c], bx = bias[channels + c];
   pdl_wait();
   if (!live) return;
   TO* o = out + (size_t)t * out_stride + c;
@@ -203,6 +203,7 @@ __global__ void mingru_step_kernel(TO* out, long long out_stride, const float* z
     return;
   }
   const float* p = zug + (size_t)t * stride + c;
+  const float old = *st;
   float a, v;
   keep_and_add<kFast>(p[0] + bz, p[col_step] + bx, a, v);
   const float S = a * old + v;

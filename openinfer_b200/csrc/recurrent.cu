@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(kThreads) recurrent_scan_kernel(ScanArgs a, in
   const int phase = a.state_phase[b];
   const float* old = a.state + (size_t)a.state_slots[b] * a.state_stride + ((size_t)phase * a.H + h) * elems;
   float* fresh = a.state + (size_t)a.state_slots[b] * a.state_stride + ((size_t)(1 - phase) * a.H + h) * elems;
+  pdl_wait();    // ahead of it the metadata alone: the old state may be what the kernel before leaves behind
   float C[kE][R], nn[R];
   float m = 0.f;
 #pragma unroll
@@ -450,7 +451,6 @@ __global__ void __launch_bounds__(kThreads) recurrent_scan_kernel(ScanArgs a, in
       a.out[(size_t)(first_row + my_row) * a.ld_out + (size_t)h * V + c0 + my_col] = kGates ? num[0] / (fmaxf(fabsf(den[0]), bound) + 1e-6f) : num[0];
     }
   };
-  pdl_wait();    // the old state's copy is the step before's: only the records and values are this step's
   request(0, 0);
   int turn = 0;
   for (int t0 = 0; t0 < n_rows; t0 += chunk, turn ^= 1) {      // chunk: a multiple of four
@@ -506,6 +506,7 @@ __global__ void __launch_bounds__(kThreads) delta_channel_scan_kernel(ScanArgs a
   const int phase = a.state_phase[b];
   const float* old = a.state + (size_t)a.state_slots[b] * a.state_stride + ((size_t)phase * a.H + h) * D * V;
   float* fresh = a.state + (size_t)a.state_slots[b] * a.state_stride + ((size_t)(1 - phase) * a.H + h) * D * V;
+  pdl_wait();    // ahead of it the metadata alone: the old state may be what the kernel before leaves behind
   float C[kE][R];
 #pragma unroll
   for (int e = 0; e < kE; ++e)
@@ -620,7 +621,6 @@ __global__ void __launch_bounds__(kThreads) delta_channel_scan_kernel(ScanArgs a
         for (int i = 0; i < R; ++i) C[e][i] += k[i] * d[e][u];
     }
   };
-  pdl_wait();    // the old state's copy is the step before's: only the records and values are this step's
   request(0, 0);
   int turn = 0;
   for (int t0 = 0; t0 < n_rows; t0 += chunk, turn ^= 1) {      // chunk: a multiple of four, so that runs do not straddle it
@@ -671,6 +671,7 @@ __global__ void __launch_bounds__(kThreads) delta_head_scan_kernel(ScanArgs a, i
   const int phase = a.state_phase[b];
   const float* old = a.state + (size_t)a.state_slots[b] * a.state_stride + ((size_t)phase * a.H + h) * D * V;
   float* fresh = a.state + (size_t)a.state_slots[b] * a.state_stride + ((size_t)(1 - phase) * a.H + h) * D * V;
+  pdl_wait();    // ahead of it the metadata alone: the old state may be what the kernel before leaves behind
   float C[kE][R];
 #pragma unroll
   for (int e = 0; e < kE; ++e)
@@ -697,7 +698,6 @@ __global__ void __launch_bounds__(kThreads) delta_head_scan_kernel(ScanArgs a, i
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  pdl_wait();    // the old state's copy is the step before's: only the records and values are this step's
   request(0, 0);
   int turn = 0;
   for (int t0 = 0; t0 < n_rows; t0 += chunk, turn ^= 1) {      // chunk: a multiple of four, so that runs do not straddle it
@@ -903,7 +903,7 @@ OI_API int oi_recurrent_scan(int mode, const float* qkv, long long ld_qkv, int q
   OI_CHECK_LAUNCH();
   // Requests of several rows in plain stream order: launched early, the few long-lived blocks would be packed onto the SMs that
   // the kernel before frees first and share their issue slots (measured 2.1 against 0.9 ms for 2,048 rows). Single rows have no
-  // such loop: launched early they fetch the old state while the records are formed.
+  // such loop: launched early they find their place while the records are formed.
   const bool single = tokens == requests;
   if (mode == kDeltaHeadDecay) {
     const int rows = D <= 128 ? 16 : (D <= 256 ? 8 : 4);       // per buffer: two buffers of at most 19 KB

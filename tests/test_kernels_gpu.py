@@ -1382,6 +1382,62 @@ def test_router_rows_of_a_large_step(E, scoring, groups, keep, K):
 
 
 # ------------------------------------------------------------------------------------------------ recurrences
+@pytest.mark.parametrize("kind", ["matrix_memory", "gated_delta", "delta_head", "linear_decay", "filter", "min_gru"])
+def test_recurrent_states_of_steps_in_a_row(kind):
+    """Steps of single rows that follow one another with no other kernel between them: each starts from the state that the one
+    before leaves behind. Bit for bit as with a wait for the GPU after every step."""
+    from types import SimpleNamespace
+
+    from openinfer_b200.kernels import ops
+    torch.manual_seed(11)
+    B, steps, H, D, V, C, taps = 6, 24, 4, 128, 128, 1024, 4
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ctxs = [SimpleNamespace(cu_seqlens=torch.arange(B + 1, **i32), token_req=torch.arange(B, **i32), state_slots=torch.arange(B, **i32),
+                            state_phase=torch.full((B,), phase, **i32), num_requests=B, decode_only=True, q_lens_host=[1] * B) for phase in (0, 1)]
+    codes = {"matrix_memory": ops.SCAN_MATRIX_MEMORY, "gated_delta": ops.SCAN_GATED_DELTA, "linear_decay": ops.SCAN_LINEAR_DECAY,
+             "delta_head": ops.SCAN_DELTA_HEAD_DECAY}
+    if kind == "filter":
+        xs, state = torch.randn(steps, B, C, device=DEV), torch.randn(B, 2, taps - 1, C, device=DEV)
+        w, outs = torch.randn(C, taps, device=DEV), torch.empty(steps, B, C, device=DEV)
+
+        def step(s, st):
+            ops.short_conv(outs[s], xs[s], w, st, ctxs[s % 2].cu_seqlens, ctxs[s % 2].token_req, ctxs[s % 2].state_slots, ctxs[s % 2].state_phase)
+    elif kind == "min_gru":
+        xs, state = torch.randn(steps, B, 3 * C, device=DEV), torch.randn(B, C, device=DEV)
+        bias, outs = torch.randn(2, C, device=DEV), torch.empty(steps, B, C, device=DEV)
+
+        def step(s, st):
+            ops.mingru_scan(outs[s], xs[s], C, bias, st, ctxs[0])
+    else:
+        memory, delta = kind == "matrix_memory", kind == "gated_delta"
+        xs, gates = torch.randn(steps, B, 2 * H * D + H * V, device=DEV), torch.randn(steps, B, 2 * H, device=DEV)
+        decay = torch.randn(steps, B, H * D, device=DEV)
+        state = torch.randn(B, 2, H, D * V + (D + 1 if memory else 0), device=DEV) * 0.3
+        if memory:
+            state[..., -1].abs_()
+        p0 = (torch.randn(H * D if delta else H, device=DEV) * 0.3).sigmoid()
+        p1, outs = torch.randn(H, device=DEV) * 0.3, torch.empty(steps, B, H * V, device=DEV)
+        source = xs.clone()        # (the linear decay turns the values into their silu in place)
+
+        def step(s, st):
+            ops.recurrent_scan(codes[kind], outs[s], xs[s], (0, H * D, 2 * H * D), gates[s], (0, H), st, ctxs[s % 2], H, H, D, V,
+                               p0=p0, p1=p1, decay=decay[s] if delta else None, cap=15.0, q_scale=D ** -0.5)
+    results = []
+    for wait in (True, False):
+        if kind not in ("filter", "min_gru"):
+            xs.copy_(source)
+        st = state.clone()
+        outs.zero_()
+        torch.cuda.synchronize()
+        for s in range(steps):
+            step(s, st)
+            if wait:
+                torch.cuda.synchronize()
+        results.append((outs.clone(), st))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    assert bool(results[0][0].isfinite().all()) and bool((results[0][0][-1] != 0).any())
+
+
 @pytest.mark.parametrize("mode", ["matrix_memory", "gated_delta", "linear_decay"])
 @pytest.mark.parametrize("D,V", [(5, 7), (32, 33), (33, 8), (64, 100), (100, 64), (128, 130), (132, 9), (256, 32), (300, 17)])
 def test_recurrent_scan_runs_of_rows(mode, D, V):
