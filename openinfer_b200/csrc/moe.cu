@@ -640,6 +640,7 @@ constexpr int kFewPairs = 64, kFewThreads = 256, kFewBlocks = 2, kFewStages = 5;
 constexpr int kFewStage = 4 * 32;                                    // 16-byte words of a warp's stage: four rows, a word a lane
 constexpr int kFewRing = kFewThreads / 32 * kFewStages * kFewStage * 16;
 constexpr int kFewInputs = 24 * 1024;                                // bytes of input rows, where one takes no more
+constexpr int kFewMostInputs = 144 * 1024, kGemvMostInputs = 200 * 1024;      // and the longest row there is room for
 
 __device__ __forceinline__ void few_cp16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -871,7 +872,11 @@ int launch_few(const T* A, long long lda, int a_div, const T* W, TO* out, long l
                float limit, int act, cudaStream_t s) {
   constexpr int kVec = 16 / (int)sizeof(T);
   const long long stride = (long long)(kGlu ? 2 : 1) * N * K;
-  if (K % kVec != 0 || (uintptr_t)W % 16 != 0) {
+  if (K % kVec != 0 || (uintptr_t)W % 16 != 0 || (long long)K * (int)sizeof(T) > kFewMostInputs) {
+    OI_REQUIRE((long long)K * 4 <= kGemvMostInputs, "moe_experts: rows of %d numbers, at most %d in steps of few rows", K, kGemvMostInputs / 4);
+    static const cudaError_t gemv_allowed =
+        cudaFuncSetAttribute(moe_gemv_kernel<T, TO, kGlu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvMostInputs);
+    OI_CHECK_CUDA(gemv_allowed);
     oi_launch(moe_gemv_kernel<T, TO, kGlu>, dim3(pairs, (N + 15) / 16), 128, (size_t)K * 4, s, A, lda, a_div, W, stride, out, ld_out, ids, E, N, K,
               limit, act);
     OI_CHECK_LAUNCH();
@@ -880,7 +885,7 @@ int launch_few(const T* A, long long lda, int a_div, const T* W, TO* out, long l
   const int fits = kFewInputs / (K * (int)sizeof(T)), at_once = fits < 1 ? 1 : (fits < 4 ? fits : 4);
   const size_t smem = kFewRing + (size_t)at_once * K * sizeof(T);
   auto kernel = moe_few_rows_kernel<T, TO, kGlu>;
-  static const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewRing + 48 * 1024);
+  static const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewRing + kFewMostInputs);
   OI_CHECK_CUDA(allowed);
   const bool x_vec = (uintptr_t)A % 16 == 0 && lda % kVec == 0;
   oi_launch(kernel, 148 * kFewBlocks, kFewThreads, smem, s, A, lda, a_div, W, stride, out, ld_out, ids, pairs, E, N, K, limit, act, at_once,
@@ -1062,7 +1067,7 @@ OI_API int oi_moe_experts(const void* x, int dtype, long long ldx, const void* w
   if (rows == 0) return OI_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const int pairs = rows * top, max_tiles = oi_moe_max_tiles(pairs, E);
-  if (oi_moe_small(pairs, E) && (size_t)(W > F ? W : F) * sizeof(float) <= 48 * 1024) {
+  if (oi_moe_small(pairs, E)) {      // whatever the widths: such a step's pairs have not been grouped (see the routes above)
     int rc = OI_OK;
     if (dtype == OI_F32) {
       rc = launch_few<float, float, true>((const float*)x, ldx, top, (const float*)w_gate_up, (float*)act, F, ids, pairs, E, F, W, limit, glu, s);

@@ -1347,6 +1347,33 @@ def test_experts_of_few_rows_add_in_float32(dtype, rows, W, F, E):
     assert torch.equal(out, lanes[..., 0])
 
 
+@pytest.mark.parametrize("W,F", [(72, 12296), (12296, 40), (40, 12301), (16, 36872), (12290, 24)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_experts_of_few_rows_and_wide_ones(dtype, W, F):
+    """A step of few rows is never grouped: widths beyond 12,288 (48 KB of float32) take the kernels of few rows too, aligned or not, and
+    what does not fit beside a ring of copies the kernel without one. Rows longer than shared memory are refused."""
+    from openinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(W + F)
+    rows, E, top = 5, 6, 2
+    x = torch.randn(rows, W, generator=g).to(dtype).to(DEV)
+    gate_up = (torch.randn(E, 2 * F, W, generator=g) * W ** -0.5).to(dtype).to(DEV)
+    down = (torch.randn(E, W, F, generator=g) * F ** -0.5).to(dtype).to(DEV)
+    table = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(rows)])
+    routing = ops.moe_route_table(torch.arange(rows, dtype=torch.int32, device=DEV), table.to(torch.int32).to(DEV), E)
+    out = ops.moe_experts(x, gate_up, down, routing, 0.0, act="silu").double()
+    ref, bound = _experts_reference(x, gate_up, down, routing[0].view(rows, top), routing[1].view(rows, top))
+    assert ((out - ref).abs() <= bound).all()
+
+
+def test_experts_of_few_rows_too_wide():
+    from openinfer_b200.kernels import ops
+    from openinfer_b200.kernels.lib import KernelError
+    x, gate_up, down = (torch.zeros(s, device=DEV) for s in ((1, 8), (2, 2 * 51204, 8), (2, 8, 51204)))
+    routing = ops.moe_route_table(torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(1, 1, dtype=torch.int32, device=DEV), 2)
+    with pytest.raises(KernelError):
+        ops.moe_experts(x, gate_up, down, routing, 0.0, act="silu")
+
+
 @pytest.mark.parametrize("rows,E,top", [(1, 4, 2), (7, 16, 2), (20, 40, 3), (40, 3, 2), (300, 5, 2)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_experts_named_twice_by_a_table(dtype, rows, E, top):
