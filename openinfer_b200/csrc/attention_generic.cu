@@ -1,6 +1,6 @@
 // Paged causal attention, general form: any head_dim that is a multiple of 8 (up to 512), any
 // number of heads and groups, an optional window or chunks, float32 or bfloat16 storage; prompt portions
-// and single decoded tokens alike. One warp per (token, query head).
+// and single decoded tokens alike. A block of eight warps per token and query head, or two heads of a kv head together.
 //
 // s[i,j] = (q_i . k_j) * scale for first_visible(pos_i) <= j <= pos_i (and j among the sequence's kept first keys),
 // online softmax in float32,
@@ -10,7 +10,7 @@
 // in the batch, so a row's result does not depend on how the batch was cut.
 //
 // What bounds it is latency: a lane's dot product is one chain over a key of its own (512 bytes at 128 float32 numbers), so
-// the loads of eight pieces are in flight before their products, and a row's key tiles run side by side. One warp a row with
+// the loads of up to sixteen 16-byte pieces (see kAhead) are in flight before their products, and a row's key tiles run side by side. One warp a row with
 // one load in flight took 255 us a layer for 2 rows of 200 keys and 16 heads of float32, 152 us for a prompt of 355 rows; now
 // 12.7 us and 79.8 us (B200).
 //

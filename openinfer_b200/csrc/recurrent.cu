@@ -14,7 +14,7 @@
 //
 // Prompts and single decoded tokens take the same two launches. A first kernel forms, for all rows at once, what does
 // not depend on earlier rows (gates, decays, unit vectors); then block (request, head, slice of value columns) walks the
-// request's rows of the step in order, its slice of C in registers (a column's D numbers spread over 4 to 16 lanes), the
+// request's rows of the step in order, its slice of C in registers (a column's D numbers spread over 8 to 32 lanes), the
 // rows' records staged in shared memory a chunk at a time (cp.async, two buffers), so that the loop over rows is the recurrence alone. The state
 // lives in two copies that take turns ([slots][2][heads][elems], C stored column by column, then n and m): a step reads
 // copy state_phase[request] and leaves the other, so no block reads what another writes. Everything is float32: the
@@ -65,8 +65,8 @@ __device__ __forceinline__ float gate_value(float z, int act) {
 __device__ __forceinline__ float softplus_f(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
 // Everything of a row that does not depend on the rows before it, one warp per (row, head), so that the scan's loop is
-// the recurrence alone. Record of rec >= 3 D + 2 floats: keys [D], queries [D], decays [D], two scalars, padding.
-//   matrix memory: keys as they are, queries times q_scale, (no decays), the log gates i and f
+// the recurrence alone. Record of rec >= 3 D + 2 floats: keys [D], queries [D], [D] that these modes leave unused, two scalars, padding.
+//   matrix memory: keys as they are, queries times q_scale, the log gates i and f
 //   linear decay:  silu of the keys, silu of the queries times q_scale; the head's values get their silu in place
 template <int kMode>
 __global__ void recurrent_prepare_kernel(ScanArgs a) {
@@ -292,12 +292,6 @@ __device__ __forceinline__ float lanes_sum(float v) {
   return v;
 }
 
-// Block (request, head, slice of 2 kThreads / kLanes value columns): the request's rows of the step in order, up to four at a
-// time, the slice of C in registers (the D numbers of two columns spread over kLanes lanes, R of each a lane), the rows' records
-// staged in shared memory a chunk at a time. Two columns share what is read of a row, and the sums over the lanes of four rows
-// are formed by halving. Bound by issue slots (0.75 instructions a clock of a scheduler with one warp). Four requests of up to
-// 1,500 rows, 8 heads, with the records: matrix memory 1,131 -> 820 us with 128 keys and 256 values; linear attention, up to 2,000
-// rows, 642 -> 468 us. (A lane's read-out in two sums instead of four takes 2 to 3 % less, and loses precision.)
 // Which key channel register i of lane j holds, and a row's D numbers into a thread's R registers. kVec4 (D a multiple of
 // four): a lane holds runs of four neighbours, d = 4 (j + (i / 4) kLanes) + i % 4, and reads them 16 bytes at a time;
 // otherwise d = j + i kLanes.
@@ -323,6 +317,12 @@ __device__ __forceinline__ void load_channels(float (&dst)[R], const float* __re
   }
 }
 
+// Block (request, head, slice of 2 kThreads / kLanes value columns): the request's rows of the step in order, up to four at a
+// time, the slice of C in registers (the D numbers of two columns spread over kLanes lanes, R of each a lane), the rows' records
+// staged in shared memory a chunk at a time. Two columns share what is read of a row, and the sums over the lanes of four rows
+// are formed by halving. Bound by issue slots (0.75 instructions a clock of a scheduler with one warp). Four requests of up to
+// 1,500 rows, 8 heads, with the records: matrix memory 1,131 -> 820 us with 128 keys and 256 values; linear attention, up to 2,000
+// rows, 642 -> 468 us. (A lane's read-out in two sums instead of four takes 2 to 3 % less, and loses precision.)
 template <int kMode, int kLanes, int R, bool kVec4>
 __global__ void __launch_bounds__(kThreads) recurrent_scan_kernel(ScanArgs a, int chunk) {
   // (no early trigger: the blocks of the kernel behind this one would wait on the SMs this latency-bound loop needs)

@@ -9,8 +9,9 @@
 // stream; here the caller supplies one uniform number per row (made from the request's own seed
 // and step, so a row's draw does not depend on its place in the batch) and the kernel walks the
 // cumulative distribution in vocabulary order. Thresholds are found by radix selection on the bit
-// pattern of the (non-negative) probabilities, over the few thousand largest of them where that
-// suffices (see sample_kernel), so no sort and no scratch beyond one float per vocabulary entry and row.
+// pattern of the (non-negative) probabilities (sample_kernel, with no scratch beyond one float per
+// vocabulary entry and row), or by a sort of the few thousand largest of them where these suffice
+// (sample_cluster_kernel, in shared memory).
 #include <cooperative_groups.h>
 
 #include "common.cuh"

@@ -137,7 +137,7 @@ DECODE_LONG_CONTEXT = 12288
 DECODE_VERY_LONG_CONTEXT = 24576   # and from here up to 128: batch 1 at 32,768 keys 240 against 229, at 65,536 206 against 188
 DECODE_VERY_LONG_SPLITS = 128
 DECODE_MIN_KEYS_PER_SPLIT = 32
-DECODE_KEYS_PER_RECORDED_SPLIT = 64   # of a recorded step's capacity: its rows hold half of that and more
+DECODE_KEYS_PER_RECORDED_SPLIT = 64   # of a recorded step's capacity: above the smallest one its rows hold half of that and more
 DECODE_MAX_GROUP = 16
 _SM_COUNT = None
 
