@@ -30,18 +30,32 @@ bool tma_ok(const void* x, long long ldx, const void* w, long long ldw, int K) {
   return K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
 }
 
+// This host thread launches a step whose experts are chosen by scores (oi_streamed_products).
+thread_local int t_streamed = 0;
+
 // How many K slices (CTAs per cluster) the streaming kernel uses: one when the tiles of 128 weight rows alone
-// fill the GPU, else the fewest slices that give every SM a CTA, each slice at least two k blocks long.
+// fill the GPU, else the fewest slices that give every SM a CTA, each slice at least two k blocks long, while the CTAs are
+// no more than 256: two fit on an SM, but clusters of 4 or 8 do not find room on all of them at once.
 // Measured on B200 at M = 8 (us, inside a CUDA graph): N 6144 K 4096: 14.2 with 4 slices (16.1 with 2, 17.0
 // with 8); N 4096 K 4096: 11.1 with 8 (11.8 with 4); N 4096 K 12288: 20.9 with 8 (22.1 with 4); N 24576 and
-// N 151936: one slice (34.4 and 188).
+// N 151936: one slice (34.4 and 188). With the norm kernel before it: N 4608 K 2048: 7.6 with 4 slices (10.2 with 8, 288
+// CTAs); N 9216 K 2048: 11.5 with 2 (14.3 with 4, 288 CTAs).
 int stream_slices(int N, int K) {
   const int tiles = (N + 127) / 128, num_kb = (K + 63) / 64;
   int c = 1;
-  while (c < 8 && tiles * c < sm_count() && num_kb / (2 * c) >= 2) c *= 2;
+  while (c < 8 && tiles * c < sm_count() && (tiles * 2 * c <= 256 || t_streamed) && num_kb / (2 * c) >= 2) c *= 2;
   if (g_opt[OI_OPT_FORCE_SLICES] > 0) c = g_opt[OI_OPT_FORCE_SLICES];
   while (c > 1 && (c - 1) * ((num_kb + c - 1) / c) >= num_kb) c /= 2;   // no slice may be left without a k block
   return c;
+}
+
+// Whether gemm_few.cu takes a decode product: rows of up to 3,072 (figures there); longer ones, which x's rows still fit, only
+// where 148 CTAs take all of W at a time (N 2048 K 6144 6.9 us against the streaming kernel's 9.1 at 8 rows): all of x has to reach
+// every SM, and beside other long streams nothing is left of it (N 4096 K 4096 11.4 against 9.6 at 16 rows; Qwen3-8B sizes at 8
+// requests 68.2 against 68.4 ms). Nor the longest streams: N 32768 K 1024 15.0 against 14.3 at 16 rows, 13.3 against 13.6 at one.
+bool few_takes(const void* x, long long ldx, const void* W, long long ldw, int M, int N, int K) {
+  return !t_streamed && g_opt[OI_OPT_FORCE_SLICES] == 0 && K >= 64 && K % 64 == 0 && K <= oi_gemm_few_max_k(M) &&
+         N <= (K <= 3072 ? 24576 : 16 * 148) && ldx % 16 == 0 && ldw % 8 == 0 && (uintptr_t)x % 32 == 0 && (uintptr_t)W % 16 == 0;
 }
 
 // K slices of the mma.sync decode product, 0 if it does not take the shape (a slice's activations must fit in
@@ -70,7 +84,7 @@ int linear_bf16(void* out, int out_dtype, long long ldc, const void* x, long lon
   const int decode_gemm = g_opt[OI_OPT_DECODE_GEMM];
   if (M <= kDecodeMaxRows) {
     if (decode_gemm == 0 && tma)
-      return oi_gemm_stream(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, stream_slices(N, K), OI_ACT_NONE, stream);
+      return oi_decode_product(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, 0, OI_ACT_NONE, 0.f, 0.f, stream);
     if (decode_gemm <= 1 && M <= kSkinnyMaxRows && tma && K >= 32) {
       const int c = skinny_slices(K);
       if (c) return oi_gemm_skinny(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, 0, 0, c, stream);
@@ -106,6 +120,21 @@ OI_API int oi_configure(int option, int value) {
 OI_API int oi_option(int option) { return option >= 0 && option < OI_OPT_COUNT ? g_opt[option] : -1; }
 
 OI_API int oi_stream_slices(int N, int K) { return stream_slices(N, K); }
+
+OI_API int oi_streamed_products(int on) {
+  const int was = t_streamed;
+  t_streamed = on;
+  return was;
+}
+
+OI_API int oi_decode_product(void* out, int out_dtype, long long ldc, const void* x, long long ldx, const void* W, long long ldw,
+                             int M, int N, int K, int glu, int act, float p0, float p1, void* stream) {
+  if (few_takes(x, ldx, W, ldw, M, N, K)) return oi_gemm_few(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, glu, act, p0, p1, stream);
+  const int c = stream_slices(N, K);
+  if (glu) return oi_gemm_stream_glu(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, c, act, p0, stream);
+  if (act != OI_ACT_NONE) return oi_gemm_stream_unary(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, c, act, p0, p1, stream);
+  return oi_gemm_stream(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, c, OI_ACT_NONE, stream);
+}
 
 OI_API int oi_linear(void* out, int out_dtype, long long ldc, const void* x, int x_dtype, long long ldx, const void* W,
                      int w_dtype, long long ldw, int M, int N, int K, void* stream) {
@@ -152,8 +181,7 @@ OI_API int oi_gated_mlp(void* out, const void* x, int dtype, int M, int hidden, 
     else
       OI_TRY(oi_gemm_tcgen05(act_buf, OI_BF16, inter, x, hidden, w_gate_up, hidden, M, 2 * inter, hidden, tile, act, stream));
   } else if (fusion == 1) {
-    OI_TRY(oi_gemm_stream(act_buf, OI_BF16, inter, x, hidden, w_gate_up, hidden, M, 2 * inter, hidden,
-                          stream_slices(2 * inter, hidden), act, stream));
+    OI_TRY(oi_decode_product(act_buf, OI_BF16, inter, x, hidden, w_gate_up, hidden, M, 2 * inter, hidden, 1, act, 0.f, 0.f, stream));
   } else {
     OI_REQUIRE(gate_up_buf != nullptr, "gated_mlp: this shape needs the gate|up scratch buffer");
     OI_TRY(oi_linear(gate_up_buf, dtype, 2 * inter, x, dtype, hidden, w_gate_up, w_dtype, hidden, M, 2 * inter, hidden, stream));
@@ -170,8 +198,7 @@ OI_API int oi_dense_mlp(float* out, const void* x, int dtype, int M, int hidden,
   // the activation in the up-projection's epilogue where a hand-written product takes the shape, else on its own
   const bool fusable = dtype == OI_BF16 && w_up_dtype == OI_BF16 && tma_ok(x, hidden, w_up, hidden, hidden);
   if (fusable && !g_opt[OI_OPT_BATCH_INVARIANT] && M <= kDecodeMaxRows && g_opt[OI_OPT_DECODE_GEMM] == 0) {
-    OI_TRY(oi_gemm_stream_unary(z_buf, dtype, inter, x, hidden, w_up, hidden, M, inter, hidden, stream_slices(inter, hidden),
-                                OI_ACT_XIELU, a_p, a_n, stream));
+    OI_TRY(oi_decode_product(z_buf, dtype, inter, x, hidden, w_up, hidden, M, inter, hidden, 0, OI_ACT_XIELU, a_p, a_n, stream));
   } else if (fusable && (M >= kFusedMinRows || g_opt[OI_OPT_BATCH_INVARIANT])) {   // 33..127 rows: the library's product is faster
     const int pairs = !g_opt[OI_OPT_BATCH_INVARIANT] && M >= g_opt[OI_OPT_PAIR_MIN_ROWS] && (hidden > 2048 || M >= 2048);
     OI_TRY(oi_gemm_tcgen05_unary(z_buf, dtype, inter, x, hidden, w_up, hidden, M, inter, hidden, pairs, OI_ACT_XIELU, a_p, a_n, stream));

@@ -288,6 +288,12 @@ OI_API int oi_gemm_stream_unary(void* out, int out_dtype, long long ldc, const v
        long long ldw, int M, int N, int K, int cluster_size, int act, float p0, float p1, void* stream);
 OI_API int oi_gemm_stream_status(int* status);
 
+// gemm_few.cu
+OI_API int oi_gemm_few(void* out, int out_dtype, long long ldc, const void* x, long long ldx, const void* W, long long ldw, int M,
+                       int N, int K, int glu, int act, float p0, float p1, void* stream);
+OI_API int oi_gemm_few_max_k(int M);
+OI_API int oi_gemm_few_status(int* status);
+
 // gemm_tcgen05.cu
 OI_API int oi_gemm_tcgen05(void* C, int c_dtype, long long ldc, const void* A, long long lda, const void* W, long long
        ldw, int M, int N, int K, int tile_n, int act, void* stream);
@@ -342,7 +348,7 @@ OI_API int oi_library_gemm(void* out, int out_dtype, long long ldc, const void* 
 // Options of the dispatch (oi_configure): values are ints.
 enum : int {
   OI_OPT_BATCH_INVARIANT = 0,   // 1: every choice depends on the request alone (one product kernel for all shapes)
-  OI_OPT_DECODE_GEMM = 1,       // products of up to 32 rows: 0 streaming tcgen05 kernel, 1 mma.sync kernel, 2 library
+  OI_OPT_DECODE_GEMM = 1,       // products of up to 32 rows: 0 gemm_few.cu and the streaming tcgen05 kernel, 1 mma.sync kernel, 2 library
   OI_OPT_PREFILL_GEMM = 2,      // plain products of more rows: 0 library, 1 the pair kernel of gemm_tcgen05.cu
   OI_OPT_FORCE_SLICES = 3,      // > 0: K slices of the decode products, whatever the shape (measurements)
   OI_OPT_PAIR_MIN_ROWS = 4,     // rows from which the fused gate/up product uses pairs of CTAs
@@ -356,6 +362,14 @@ OI_API int oi_option(int option);
 // y[M, N] = x[M, K] W[N, K]^T by the kernel that the operand types, the shape and the options select.
 OI_API int oi_linear(void* out, int out_dtype, long long ldc, const void* x, int x_dtype, long long ldx, const void* W,
        int w_dtype, long long ldw, int M, int N, int K, void* stream);
+// A product of up to 32 rows, bfloat16 operands that TMA can fetch: gemm_few.cu where it is the faster one, else
+// gemm_stream.cu. glu, act, p0, p1 as oi_gemm_few has them.
+OI_API int oi_decode_product(void* out, int out_dtype, long long ldc, const void* x, long long ldx, const void* W, long long ldw,
+                             int M, int N, int K, int glu, int act, float p0, float p1, void* stream);
+// on != 0: the products that the calling host thread launches from here on keep the streaming kernel and its K slices (a
+// step whose experts are chosen by scores: the last bits of the products ahead of a router decide its near ties, and
+// such a model keeps the choices it has always made). Returns what it was.
+OI_API int oi_streamed_products(int on);
 // How many K slices the streaming product uses for a shape (what oi_linear passes to oi_gemm_stream).
 OI_API int oi_stream_slices(int N, int K);
 

@@ -1,7 +1,7 @@
 """Numeric policy: whether a request's results may depend, at rounding level, on what else is in the batch.
 
-By default the kernels are chosen for speed by the shape of the whole step: the streaming product up to
-32 rows and the library beyond, more or fewer key slices per decode row depending on how many rows there
+By default the kernels are chosen for speed by the shape of the whole step: the products of few rows up to 16, the
+streaming product up to 32 rows and the library beyond, more or fewer key slices per decode row depending on how many rows there
 are, tiles of 64 or 128 query rows, the rotation inside or in front of the attention kernel. Every choice
 computes the same thing in float32 but may round differently, so a request's logits agree between batches
 only "beyond rounding".
@@ -20,6 +20,8 @@ bits when they cut prompts alike (the same ``max_prefill_tokens``).
 """
 from __future__ import annotations
 
+from contextlib import contextmanager
+
 _BATCH_INVARIANT = False
 INVARIANT_DECODE_SPLITS = 16
 
@@ -34,3 +36,16 @@ def set_batch_invariant(on: bool) -> None:
 
 def batch_invariant() -> bool:
     return _BATCH_INVARIANT
+
+
+@contextmanager
+def streamed_products():
+    """While it lasts, this thread's decode products keep the streaming kernel and its K slices: for steps whose experts are
+    chosen by scores, where the last bits of the products ahead of a router decide near ties (``oi_streamed_products``)."""
+    from . import lib
+    L = lib.load()
+    was = L.oi_streamed_products(1)
+    try:
+        yield
+    finally:
+        L.oi_streamed_products(was)

@@ -62,9 +62,9 @@ class GatedMlp(FeedForward):
                 or x.data_ptr() % 16 or policy.batch_invariant()):
             return False
         if M <= 32 and N % 128 == 0:
-            _lib.check(L.oi_gemm_stream_glu(act.data_ptr(), 1, act.stride(0), x.data_ptr(), x.stride(0), self.w_gate_up.data_ptr(),
-                                            self.w_gate_up.stride(0), M, N, K, L.oi_stream_slices(N, K), self.act_code, float(s.limit),
-                                            _lib.current_stream()), "gemm_stream_glu")
+            _lib.check(L.oi_decode_product(act.data_ptr(), 1, act.stride(0), x.data_ptr(), x.stride(0), self.w_gate_up.data_ptr(),
+                                           self.w_gate_up.stride(0), M, N, K, 1, self.act_code, float(s.limit), 0.0,
+                                           _lib.current_stream()), "decode_product")
             return True
         if M >= 128 and N % 256 == 0:
             _lib.check(L.oi_gemm_tcgen05_glu(act.data_ptr(), act.stride(0), x.data_ptr(), x.stride(0), self.w_gate_up.data_ptr(),

@@ -9,11 +9,12 @@ import torch
 
 import ctypes
 import os
+from contextlib import nullcontext
 
 from ..cache.manager import CacheManager
 from ..kernels import attention as attn_kernels
 from ..kernels import lib as _lib
-from ..kernels import native, ops
+from ..kernels import native, ops, policy
 from ..kernels.linear import ensure_library, linear
 from .base import Block, CacheBinding, Part
 from .registry import build_block, build_norm
@@ -48,6 +49,7 @@ class Model:
         self.bindings: List[CacheBinding] = []
         self.device: Optional[torch.device] = None
         self.native_step = NATIVE_STEP
+        self.routes_by_score = any(getattr(b.feed_forward, "routes_by_score", False) for b in self.blocks)
         self._native = None          # (ModelDesc, what it points to), made at the first step
         self._native_checked = False
 
@@ -202,8 +204,9 @@ class Model:
         desc = self._native_description(ctx) if self.native_step else None
         if desc is not None:
             return self._run_native(desc, ctx, row_idx)
-        h, pending = self.forward(ctx)
-        return self.logits(h, pending, row_idx) if row_idx is not None else None
+        with policy.streamed_products() if self.routes_by_score else nullcontext():
+            h, pending = self.forward(ctx)
+            return self.logits(h, pending, row_idx) if row_idx is not None else None
 
     # ------------------------------------------------------------------ the native step
     def _native_description(self, ctx):

@@ -56,6 +56,7 @@ class RoutedExperts(FeedForward):
         if self.shared is not None and not getattr(self.shared, "takes_out_dtype", False):
             raise ValueError("routed_experts: the shared expert must be able to return float32")
         self.table: Optional[torch.Tensor] = None
+        self.routes_by_score = s.routing != "table"
         self.w_router: Optional[torch.Tensor] = None
         self.w_gate_up: Optional[torch.Tensor] = None
         self.w_down: Optional[torch.Tensor] = None

@@ -1,5 +1,6 @@
 """Each CUDA kernel alone against a plain float32 statement of the same operation, at sizes
 other than the engine's (widths that are no power of two, odd row counts, every head size)."""
+import ctypes
 import math
 import random
 
@@ -1770,3 +1771,73 @@ def test_embedding_widened(hidden):
     out = torch.empty(5, hidden, device=DEV)
     ops.embedding(out, table, ids)
     assert torch.equal(out, table[ids.long()].float())
+
+
+# one stage of a row / more than one with a rest; rows of W: fewer than eight, no multiple of eight, eight a CTA (1024), more than
+# the ring holds at once (12,288 x 2,048 and 2,048 x 6,144); every number of tokens' tiles
+@pytest.mark.parametrize("M,N,K", [(1, 5, 64), (2, 13, 192), (8, 1024, 1024), (9, 1000, 1088), (16, 300, 3072), (3, 2376, 2112),
+                                   (8, 12288, 2048), (7, 2048, 6144), (16, 16384, 1024), (12, 4104, 4096)])
+@pytest.mark.parametrize("act", ["none", "xielu", "silu", "swiglu_clamp"])
+def test_gemm_few(M, N, K, act):
+    """The product of few rows against float64, into rows with a gap behind them; its results do not depend on the other rows."""
+    from openinfer_b200.kernels import lib as klib
+    L = klib.load()
+    glu = act in ("silu", "swiglu_clamp")
+    N = -(-N // 128) * 128 if glu else N
+    g = torch.Generator(device=DEV).manual_seed(N + K + M)
+    x = torch.randn(M, K + 16, device=DEV, generator=g).to(torch.bfloat16)[:, :K]
+    w = (torch.randn(N, K + 8, device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)[:, :K]
+    ref = x.double() @ w.double().t()
+    code, p0, p1 = {"none": (0, 0.0, 0.0), "xielu": (3, 0.8, 0.9), "silu": (1, 0.0, 0.0), "swiglu_clamp": (4, 0.5, 0.0)}[act]
+    if act == "xielu":
+        ref = torch.where(ref > 0, p0 * ref * ref, p1 * (torch.expm1(ref) - ref)) + 0.5 * ref
+    if glu:
+        a, b = ref.view(M, N // 128, 2, 64).unbind(2)
+        if act == "silu":
+            ref = a * torch.sigmoid(a) * b
+        else:
+            a, b = a.clamp(max=p0), b.clamp(-p0, p0)
+            ref = a * torch.sigmoid(1.702 * a) * (b + 1.0)
+        ref = ref.reshape(M, N // 2)
+    cols = ref.shape[1]
+
+    def product(rows, out):
+        klib.check(L.oi_gemm_few(out.data_ptr(), 1 if out.dtype == torch.bfloat16 else 0, out.stride(0), rows.data_ptr(), rows.stride(0),
+                                 w.data_ptr(), w.stride(0), rows.shape[0], N, K, int(glu), code, p0, p1,
+                                 torch.cuda.current_stream().cuda_stream), "gemm_few")
+
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.full((M + 1, cols + 3), 7.0, device=DEV, dtype=dtype)
+        product(x, out[:, :cols])
+        # sums of K terms of size 1 / sqrt(K) in float32 (the exponentials are good to 2 ulp), one rounding to the result's type
+        tol = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -18) * (1.0 + ref.abs().max().item())
+        assert (out[:M, :cols].double() - ref).abs().max().item() <= tol
+        assert (out[M] == 7.0).all() and (out[:, cols:] == 7.0).all()
+        one = torch.empty((1, cols), device=DEV, dtype=dtype)
+        product(x[M - 1:], one)
+        assert torch.equal(one[0], out[M - 1, :cols])
+    v = ctypes.c_int(0)
+    L.oi_gemm_few_status(ctypes.byref(v))
+    assert v.value == 0
+
+
+def test_gemm_few_refuses_what_it_cannot_take():
+    from openinfer_b200.kernels import lib as klib
+    from openinfer_b200.kernels import linear as lin
+    L = klib.load()
+    x, w = torch.zeros(17, 8192, device=DEV, dtype=torch.bfloat16), torch.zeros(130, 8192, device=DEV, dtype=torch.bfloat16)
+    out = torch.zeros(17, 130, device=DEV, dtype=torch.bfloat16)
+
+    def rc(M, N, K, glu=0, act=0, xoff=0, woff=0, ldx=8192, ldw=8192):
+        return L.oi_gemm_few(out.data_ptr(), 1, 130, x.data_ptr() + xoff, ldx, w.data_ptr() + woff, ldw, M, N, K, glu, act, 0.0, 0.0,
+                             torch.cuda.current_stream().cuda_stream)
+
+    for bad in (dict(M=17, N=128, K=64), dict(M=0, N=128, K=64), dict(M=9, N=128, K=6144), dict(M=8, N=128, K=8192), dict(M=8, N=128, K=96),
+                dict(M=8, N=128, K=64, xoff=16), dict(M=8, N=128, K=64, woff=8), dict(M=8, N=128, K=64, ldx=8), dict(M=8, N=128, K=64, ldw=4),
+                dict(M=8, N=130, K=64, glu=1, act=1), dict(M=8, N=128, K=64, act=1), dict(M=8, N=128, K=64, glu=1, act=3)):
+        assert rc(**bad) != 0 and b"gemm_few" in L.oi_last_error(), bad
+    # and the dispatch then uses the streaming kernel: rows of x 16 bytes off, K that is no multiple of 64, 17 rows
+    for M, K, off in ((4, 1024, 8), (4, 1000, 0), (17, 1024, 0)):
+        xx = torch.randn(M, K + 8, device=DEV).to(torch.bfloat16).flatten()[off: off + M * K].view(M, K)
+        ww = torch.randn(96, K, device=DEV).to(torch.bfloat16)
+        assert (lin.linear(xx, ww, out_dtype=torch.float32).double() - xx.double() @ ww.double().t()).abs().max().item() <= 2e-5 * K
