@@ -124,6 +124,7 @@ class CacheManager:
         self.groups: List[_Group] = []
         self.state_needs: List[StateNeed] = []
         self.state_tensors: List[object] = []
+        self._clearer = None             # on a GPU: zeroes a slot of all of them by one launch
         self.slot_pool: Optional[IdPool] = None
         self.requests: Dict[Hashable, _Request] = {}
         self._allocated = False
@@ -183,6 +184,10 @@ class CacheManager:
                 sdtype = dtype if need.dtype == "model" else torch.float32
                 shape = (max_requests, need.phases, *need.shape) if need.phases > 1 else (max_requests, *need.shape)
                 self.state_tensors.append(torch.zeros(shape, dtype=sdtype, device=device))
+            if self.state_tensors and self.state_tensors[0].is_cuda:
+                from ..kernels.ops import SlotClearer
+
+                self._clearer = SlotClearer(self.state_tensors)
         self._allocated = True
 
     # ------------------------------------------------------------------
@@ -297,8 +302,11 @@ class CacheManager:
         if request_id in self.requests:
             raise KeyError(f"request {request_id!r} is already open")
         slot = self.slot_pool.allocate(1)[0]  # raises OutOfPages when all slots are taken
-        for t in self.state_tensors:
-            t[slot].zero_()
+        if self._clearer is not None:
+            self._clearer.clear(slot)
+        else:
+            for t in self.state_tensors:
+                t[slot].zero_()
         self.requests[request_id] = _Request(tables=[[] for _ in self.groups], state_slot=slot)
         return slot
 

@@ -121,6 +121,31 @@ __global__ void copy_words_kernel(int* __restrict__ dst, const int* __restrict__
   }
 }
 
+// A request's slot in every state tensor is zeroed by one launch: blockIdx.y names the tensor, table [tensors][3] its first byte,
+// the bytes from one slot to the next and the bytes of a slot. A launch a tensor left the GPU idle while the host made them:
+// passes that open 16 requests of 8 states / 8 of 24 took 19.73 / 46.3 ms, 19.08 / 45.4 so.
+__global__ void clear_slots_kernel(const long long* __restrict__ table, long long slot) {
+  pdl_start();
+  const long long* t = table + 3 * blockIdx.y;
+  unsigned char* p = reinterpret_cast<unsigned char*>(t[0] + slot * t[1]);
+  const long long bytes = t[2], step = (long long)gridDim.x * blockDim.x, me = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (((uintptr_t)p | (uintptr_t)bytes) % 16 == 0) {
+    for (long long i = me; i < bytes / 16; i += step) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
+  } else {
+    for (long long i = me; i < bytes; i += step) p[i] = 0;
+  }
+}
+
+// max_bytes: the largest slot's bytes
+OI_API int oi_clear_slots(const long long* table, int tensors, long long max_bytes, long long slot, void* stream) {
+  OI_REQUIRE(table && tensors >= 0 && tensors <= 65535 && max_bytes >= 0 && slot >= 0, "clear_slots: bad sizes");
+  if (tensors == 0 || max_bytes == 0) return OI_OK;
+  const long long want = (max_bytes + 256 * 16 * 4 - 1) / (256 * 16 * 4);
+  oi_launch(clear_slots_kernel, dim3((unsigned)(want < 64 ? want : 64), tensors), 256, 0, (cudaStream_t)stream, table, slot);
+  OI_CHECK_LAUNCH();
+  return OI_OK;
+}
+
 OI_API int oi_copy_words(int* dst, const int* src, int n, int ids_off, int src_off, int n_ids, const int* from, int n_from,
                          void* stream) {
   OI_REQUIRE(n >= 0 && (ids_off < 0 || (src_off >= 0 && n_ids >= 0 && ids_off + n_ids <= n && src_off + n_ids <= n)),

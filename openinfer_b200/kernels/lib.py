@@ -46,6 +46,7 @@ _SIGNATURES = {
     "oi_gemm_few_status": [ctypes.POINTER(c_int)],
     "oi_decode_product": [P, I, L, P, L, P, L, I, I, I, I, I, F, F, P],
     "oi_streamed_products": [I],
+    "oi_clear_slots": [P, I, L, L, P],
     "oi_set_pdl": [I],
     "oi_gemm_stream_status": [ctypes.POINTER(c_int)],
     "oi_attention_mma": [P, I, P, I, P, P, L, I, P, I, P, P, P, I, P, I, I, I, I, I, F, I, P, P, I, I, P],

@@ -91,6 +91,25 @@ def copy_words(dst: torch.Tensor, src: torch.Tensor, n: int, *, ids_off: int = -
         L.oi_launch_fence()
 
 
+class SlotClearer:
+    """Zeroes one slot (index of the first dimension) of several contiguous tensors by one launch."""
+
+    def __init__(self, tensors) -> None:
+        self.tensors = list(tensors)               # they live as long as their addresses are used
+        _cuda(*self.tensors)
+        if any(not t.is_contiguous() for t in self.tensors):
+            raise KernelError("clear_slots: the tensors must be contiguous")
+        rows = [(t.data_ptr(), t.stride(0) * t.element_size(), t[0].numel() * t.element_size()) for t in self.tensors]
+        self.slots = min(t.shape[0] for t in self.tensors)
+        self.max_bytes = max(r[2] for r in rows)
+        self.table = torch.tensor(rows, dtype=torch.int64).to(self.tensors[0].device)
+
+    def clear(self, slot: int) -> None:
+        if not 0 <= slot < self.slots:
+            raise KernelError(f"clear_slots: slot {slot} of {self.slots}")
+        _lib.check(_lib.load().oi_clear_slots(self.table.data_ptr(), len(self.tensors), self.max_bytes, slot, _stream()), "clear_slots")
+
+
 class UploadRing:
     """Small host arrays of int32 to the device without a copy-engine operation and without making the host wait
     for the stream: a ring of pinned buffers that a kernel reads (``copy_words``), each guarded by the event of its

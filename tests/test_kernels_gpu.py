@@ -1841,3 +1841,19 @@ def test_gemm_few_refuses_what_it_cannot_take():
         xx = torch.randn(M, K + 8, device=DEV).to(torch.bfloat16).flatten()[off: off + M * K].view(M, K)
         ww = torch.randn(96, K, device=DEV).to(torch.bfloat16)
         assert (lin.linear(xx, ww, out_dtype=torch.float32).double() - xx.double() @ ww.double().t()).abs().max().item() <= 2e-5 * K
+
+
+@pytest.mark.parametrize("slots,slot", [(1, 0), (5, 2), (5, 4)])
+def test_clear_slots(slots, slot):
+    """One slot of every tensor is zeroed, whatever its size, type and alignment; the others stay."""
+    from openinfer_b200.kernels import ops
+    shapes = [((3,), torch.bfloat16), ((8,), torch.float32), ((2, 3, 7), torch.float32), ((4, 128, 128), torch.float32), ((2, 3, 4096), torch.bfloat16),
+              ((1500, 1001), torch.float32)]
+    tensors = [torch.ones((slots, *s), dtype=d, device=DEV) for s, d in shapes]
+    ops.SlotClearer(tensors).clear(slot)
+    for t in tensors:
+        assert not t[slot].any()
+        t[slot] = 1
+        assert (t == 1).all()
+    with pytest.raises(ops.KernelError):
+        ops.SlotClearer(tensors).clear(slots)
