@@ -401,6 +401,28 @@ OI_API int oi_forward_branch(const OiBranchModelDesc* m, const OiBranchStepDesc*
     results = 1;
   }
   bool low_valid = false;      // `low` holds the stream as it stands
+  // A layer's last branch joins the stream and the average over the history is formed. From the fourth result on, one average
+  // in four also adds up what the next three need of the history so far (OiDepthAhead; before that they are as short as what is left).
+  int ahead_from = 0, ahead_used = 0, ahead_have = 0;
+  auto join_averaged = [&](int i, const void* norm_w, int norm_dtype, float eps, float offset) {
+    const OiBranchLayerDesc& L = m->layers[i];
+    OiDepthAhead d = {};
+    const int left = ahead_used < ahead_have ? ahead_used++ : -1;
+    if (st->ahead && oi_branch_ahead_ok(st->h, st->branch, norm_w, st->hist, st->ahead, st->low, H, results + kDepthAhead)) {
+      if (left >= 0) {
+        d.sum = st->ahead + left * hist_stride;
+        d.from = ahead_from;
+      } else if (results >= 4) {
+        for (int q = i + 1; q < m->num_layers && d.next < kDepthAhead; ++q)
+          if (m->layers[q].depth_coef) d.coef[d.next] = m->layers[q].depth_coef, d.coef_dtype[d.next++] = m->layers[q].depth_dtype;
+        d.out = st->ahead;
+        d.stride = hist_stride;
+        ahead_from = results, ahead_used = 0, ahead_have = d.next;
+      }
+    }
+    return oi_branch_norm_add_ahead(st->h, st->branch, OI_F32, norm_w, norm_dtype, T, H, eps, offset, st->hist, hist_stride, results,
+                                    L.depth_coef, L.depth_dtype, st->low, d.from || d.next ? &d : nullptr, stream);
+  };
   for (int i = 0; i < m->num_layers; ++i) {
     const OiBranchLayerDesc& L = m->layers[i];
     OI_REQUIRE(L.attn_step >= 0 && L.attn_step < st->num_attn_steps, "forward_branch: layer %d names attention step %d of %d", i,
@@ -438,14 +460,15 @@ OI_API int oi_forward_branch(const OiBranchModelDesc* m, const OiBranchStepDesc*
     OI_REQUIRE(!averaged || (st->hist && L.depth_terms == results + 1), "forward_branch: layer %d averages %d terms, %d exist", i,
                L.depth_terms, results + 1);
     const bool has_ff = L.w_up != nullptr;
-    OI_TRY(oi_branch_norm_add(st->h, st->branch, OI_F32, L.mixer_norm_w, L.mixer_norm_dtype, T, H, L.mixer_eps, L.mixer_offset,
-                              (!has_ff && averaged) ? st->hist : nullptr, hist_stride, results, L.depth_coef, L.depth_dtype,
-                              st->low, stream));
+    if (!has_ff && averaged) OI_TRY(join_averaged(i, L.mixer_norm_w, L.mixer_norm_dtype, L.mixer_eps, L.mixer_offset));
+    else OI_TRY(oi_branch_norm_add(st->h, st->branch, OI_F32, L.mixer_norm_w, L.mixer_norm_dtype, T, H, L.mixer_eps, L.mixer_offset, nullptr,
+                                   hist_stride, results, nullptr, OI_F32, st->low, stream));
     if (has_ff) {
       OI_TRY(oi_dense_mlp(st->branch, dt == OI_F32 ? (const void*)st->h : st->low, dt, T, H, L.inter, L.w_up, L.w_up_dtype, L.w_down,
                           L.w_down_dtype, L.act_pq, L.pq_dtype, L.act_a_p, L.act_a_n, st->z, stream));
-      OI_TRY(oi_branch_norm_add(st->h, st->branch, OI_F32, L.ff_norm_w, L.ff_norm_dtype, T, H, L.ff_eps, L.ff_offset,
-                                averaged ? st->hist : nullptr, hist_stride, results, L.depth_coef, L.depth_dtype, st->low, stream));
+      if (averaged) OI_TRY(join_averaged(i, L.ff_norm_w, L.ff_norm_dtype, L.ff_eps, L.ff_offset));
+      else OI_TRY(oi_branch_norm_add(st->h, st->branch, OI_F32, L.ff_norm_w, L.ff_norm_dtype, T, H, L.ff_eps, L.ff_offset, nullptr, hist_stride,
+                                     results, nullptr, OI_F32, st->low, stream));
     }
     if (averaged) ++results;
     low_valid = st->low != nullptr;

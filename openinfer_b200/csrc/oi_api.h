@@ -251,6 +251,22 @@ OI_API int oi_gemm_stream_glu(void* out, int out_dtype, long long ldc, const voi
 OI_API int oi_gemm_tcgen05_glu(void* C, long long ldc, const void* A, long long lda, const void* W, long long ldw, int M,
        int N, int K, int pair, int act, float limit, void* stream);
 
+// Depth averages share their earlier terms: what oi_branch_norm_add_ahead starts an average from, and what it leaves of the
+// averages of the layers behind (branch_ops.cu).
+constexpr int kDepthAhead = 3;
+typedef struct {
+  const float* sum;                   // with from > 0: the terms below `from` of this average, added up [rows, hidden]
+  int from, next;                     // next: how many later averages' terms below n_prev to add up (0..3; from must be 0 then)
+  float* out;                         // ... into [next][rows, hidden], `stride` numbers apart
+  long long stride;
+  const void* coef[kDepthAhead];      // their coefficients
+  int coef_dtype[kDepthAhead];
+} OiDepthAhead;
+OI_API int oi_branch_norm_add_ahead(float* h, const void* a, int a_dtype, const void* w, int w_dtype, int rows, int hidden, float eps,
+                                    float w_offset, float* hist, long long hist_stride, int n_prev, const void* coef, int coef_dtype,
+                                    void* low, const OiDepthAhead* ahead, void* stream);
+OI_API int oi_branch_ahead_ok(const void* h, const void* a, const void* w, const void* hist, const void* sums, const void* low, int hidden,
+                              int terms);
 OI_API int oi_latent_store(void* pages, long long page_stride, int page_size, int row_elems, const void* src, long
        long src_stride, int dtype, const void* w, int w_dtype, const int* slots, int tokens, int rank, float eps,
        float w_offset, void* stream);
@@ -532,6 +548,7 @@ typedef struct OiBranchStepDesc {
   const int* state_phase;     // [requests] which copy of a two-phase state the step reads
   float* h;                   // [tokens, hidden] the stream
   float* hist;                // [num_layers + 1, tokens, hidden] or null (no layer averages)
+  float* ahead;               // [kDepthAhead, tokens, hidden]: what averages leave for later ones; or null
   void* u;                    // [tokens, hidden] what the mixer reads, in the model's type
   void* low;                  // [tokens, hidden] the stream rounded to the model's type (bfloat16 models; else null)
   void* proj;                 // [tokens, max in_cols]

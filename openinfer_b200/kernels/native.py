@@ -112,6 +112,14 @@ class BranchLayerDesc(Structure):
     ]
 
 
+DEPTH_AHEAD = 3
+
+
+class DepthAhead(Structure):
+    _fields_ = [("sum", c_void_p), ("from_", c_int), ("next", c_int), ("out", c_void_p), ("stride", c_longlong),
+                ("coef", c_void_p * DEPTH_AHEAD), ("coef_dtype", c_int * DEPTH_AHEAD)]
+
+
 class BranchModelDesc(Structure):
     _fields_ = [
         ("layers", POINTER(BranchLayerDesc)), ("embedding", c_void_p), ("final_norm_w", c_void_p), ("head", c_void_p),
@@ -126,7 +134,7 @@ class BranchStepDesc(Structure):
     _fields_ = [
         ("token_ids", c_void_p), ("attn_steps", POINTER(AttnStep)), ("want_rows", c_void_p), ("cu_seqlens", c_void_p),
         ("token_req", c_void_p), ("state_slots", c_void_p), ("state_phase", c_void_p),
-        ("h", c_void_p), ("hist", c_void_p), ("u", c_void_p), ("low", c_void_p), ("proj", c_void_p), ("mixed", c_void_p),
+        ("h", c_void_p), ("hist", c_void_p), ("ahead", c_void_p), ("u", c_void_p), ("low", c_void_p), ("proj", c_void_p), ("mixed", c_void_p),
         ("branch", c_void_p), ("z", c_void_p), ("wanted", c_void_p), ("logits", c_void_p),
         ("tokens", c_int), ("requests", c_int), ("num_attn_steps", c_int), ("num_want", c_int),
     ]
@@ -150,6 +158,8 @@ def declare(lib) -> None:
     lib.oi_forward_branch.argtypes, lib.oi_forward_branch.restype = [POINTER(BranchModelDesc), POINTER(BranchStepDesc), P], c_int
     lib.oi_launches.argtypes, lib.oi_launches.restype = [], ctypes.c_ulonglong
     lib.oi_launch_fence.argtypes, lib.oi_launch_fence.restype = [], c_int
+    lib.oi_branch_norm_add_ahead.argtypes = [P, P, I, P, I, I, I, c_float, c_float, P, L, I, P, I, P, POINTER(DepthAhead), P]
+    lib.oi_branch_norm_add_ahead.restype = c_int
     lib.oi_gemm_stream_fused.argtypes = [P, I, L, P, L, P, L, I, I, I, I, I, POINTER(StreamEpilogue), P]
     lib.oi_gemm_stream_fused.restype = c_int
 

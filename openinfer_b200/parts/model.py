@@ -371,6 +371,7 @@ class Model:
         h, branch, u = buf(H, f32), buf(H, f32), buf(H)
         low = buf(H) if dt != f32 else None
         hist = torch.empty((len(self.calls) + 1, T, H), dtype=f32, device=dev) if desc.averaged else None
+        ahead = torch.empty((native.DEPTH_AHEAD, T, H), dtype=f32, device=dev) if desc.averaged and len(self.calls) > 4 else None
         proj, mixed, z = buf(desc.max_in), buf(desc.max_mixed), buf(desc.max_inter)
         steps = (native.AttnStep * len(keys))()
         kept = []
@@ -395,7 +396,7 @@ class Model:
             token_ids=ctx.token_ids.data_ptr(), attn_steps=steps, want_rows=ptr(row_idx) if n_want else 0,
             cu_seqlens=ctx.cu_seqlens.data_ptr(), token_req=ctx.token_req.data_ptr(), state_slots=ctx.state_slots.data_ptr(),
             state_phase=ctx.state_phase.data_ptr(),
-            h=h.data_ptr(), hist=ptr(hist), u=u.data_ptr(), low=ptr(low), proj=proj.data_ptr(), mixed=mixed.data_ptr(),
+            h=h.data_ptr(), hist=ptr(hist), ahead=ptr(ahead), u=u.data_ptr(), low=ptr(low), proj=proj.data_ptr(), mixed=mixed.data_ptr(),
             branch=branch.data_ptr(), z=z.data_ptr(), wanted=ptr(wanted), logits=ptr(logits), tokens=T, requests=ctx.num_requests,
             num_attn_steps=len(keys), num_want=n_want)
         _lib.check(lib.oi_forward_branch(ctypes.byref(desc), ctypes.byref(step), _lib.current_stream()), "forward_branch")

@@ -1857,3 +1857,44 @@ def test_clear_slots(slots, slot):
         assert (t == 1).all()
     with pytest.raises(ops.KernelError):
         ops.SlotClearer(tensors).clear(slots)
+
+
+@pytest.mark.parametrize("rows,hidden", [(1, 64), (9, 2048), (700, 1028)])
+@pytest.mark.parametrize("coef_dtype", DTYPES)
+def test_depth_averages_share_their_earlier_terms(rows, hidden, coef_dtype):
+    """Averages that start from what an earlier one left: bit for bit what each forms by itself."""
+    from openinfer_b200.kernels import lib as klib
+    from openinfer_b200.kernels import native, ops
+    L = klib.load()
+    g = torch.Generator(device=DEV).manual_seed(rows + hidden)
+    n = 12
+    w = torch.randn(hidden, device=DEV, generator=g)
+    coefs = [torch.randn(j + 2, device=DEV, generator=g).to(coef_dtype) for j in range(n)]
+    branches = torch.randn(n, rows, hidden, device=DEV, generator=g)
+    first = torch.randn(rows, hidden, device=DEV, generator=g)
+    hists, hs, lows = [], [], []
+    for shared in (False, True):
+        h, hist = first.clone(), torch.full((n + 1, rows, hidden), float("nan"), device=DEV)
+        low = torch.empty(rows, hidden, device=DEV, dtype=torch.bfloat16)
+        out = torch.full((native.DEPTH_AHEAD, rows, hidden), float("nan"), device=DEV)
+        hist[0] = h
+        start = have = 0
+        for i in range(n):
+            if not shared:
+                ops.branch_norm_add(h, branches[i], w, 1e-6, history=hist, n_prev=i + 1, coef=coefs[i], low=low)
+                continue
+            d = native.DepthAhead()
+            if i < start + 1 + have and have and i > start:
+                d.sum, d.from_ = out[i - start - 1].data_ptr(), start + 1
+            else:
+                start, have = i, min(native.DEPTH_AHEAD, n - 1 - i)
+                d.next, d.out, d.stride = have, out.data_ptr(), out.stride(0)
+                for q in range(have):
+                    d.coef[q], d.coef_dtype[q] = coefs[i + 1 + q].data_ptr(), native.DTYPE_CODE[coef_dtype]
+            klib.check(L.oi_branch_norm_add_ahead(h.data_ptr(), branches[i].data_ptr(), 0, w.data_ptr(), 0, rows, hidden, 1e-6, 0.0, hist.data_ptr(),
+                                                  hist.stride(0), i + 1, coefs[i].data_ptr(), native.DTYPE_CODE[coef_dtype], low.data_ptr(),
+                                                  ctypes.byref(d), torch.cuda.current_stream().cuda_stream), "branch_norm_add_ahead")
+        hists.append(hist)
+        hs.append(h)
+        lows.append(low)
+    assert torch.equal(*hists) and torch.equal(*hs) and torch.equal(*lows)
