@@ -35,7 +35,7 @@ constexpr int kMaxTop = 32;
 
 // One warp: the choice of one row from its logits z (behind them room for scores and group scores, [E] each).
 __device__ __forceinline__ void choose(float* z, unsigned char* taken, int row, int E, int top, int* __restrict__ ids, float* __restrict__ wts,
-                                       int scoring, const float* __restrict__ correction, int n_groups, int keep_groups, float weight_scale) {
+                                       int scoring, const float* corr, int n_groups, int keep_groups, float weight_scale) {
   const int lane = threadIdx.x & 31;
   float* sc = z + E;
   float* gs = z + 2 * E;
@@ -50,7 +50,7 @@ __device__ __forceinline__ void choose(float* z, unsigned char* taken, int row, 
     for (int e = lane; e < E; e += 32) {
       const float s = scoring == 2 ? expf(z[e] - top_z) / sum : 1.f / (1.f + expf(-z[e]));
       sc[e] = s;
-      z[e] = s + (correction ? correction[e] : 0.f);
+      z[e] = s + (corr ? corr[e] : 0.f);
     }
     __syncwarp();
     if (n_groups > 1 && keep_groups < n_groups) {
@@ -87,8 +87,8 @@ __device__ __forceinline__ void choose(float* z, unsigned char* taken, int row, 
       }
     }
   }
-  float chosen_z[kMaxTop];
-  int chosen_e[kMaxTop];
+  float own_z = 0.f;               // lane j keeps the j-th choice
+  int own_e = 0;
   for (int j = 0; j < top; ++j) {
     float best = -INFINITY;
     int be = 0x7fffffff;
@@ -112,58 +112,76 @@ __device__ __forceinline__ void choose(float* z, unsigned char* taken, int row, 
     if (be >= E) be = j;          // nothing open (cannot happen with sizes the entry point accepts): still an expert that exists
     if (lane == 0) taken[be] = 1;
     __syncwarp();
-    chosen_z[j] = best;
-    chosen_e[j] = be;
+    if (lane == j) own_z = best, own_e = be;
   }
-  if (lane == 0 && scoring == 2) {
-    for (int j = 0; j < top; ++j) {
-      ids[(size_t)row * top + j] = chosen_e[j];
-      wts[(size_t)row * top + j] = sc[chosen_e[j]] * weight_scale;
-    }
-  } else if (lane == 0 && scoring == 1) {
+  const bool mine = lane < top;
+  const size_t at = (size_t)row * top + lane;
+  float weight;
+  if (scoring == 2) {
+    weight = mine ? sc[own_e] * weight_scale : 0.f;
+  } else if (scoring == 1) {
+    const float score = mine ? sc[own_e] : 0.f;
     float sum = 0.f;
-    for (int j = 0; j < top; ++j) sum += sc[chosen_e[j]];
-    for (int j = 0; j < top; ++j) {
-      ids[(size_t)row * top + j] = chosen_e[j];
-      wts[(size_t)row * top + j] = sc[chosen_e[j]] / (sum + 1e-20f);
-    }
-  } else if (lane == 0) {
-    float mx = chosen_z[0], sum = 0.f;
-    for (int j = 1; j < top; ++j) mx = fmaxf(mx, chosen_z[j]);
-    for (int j = 0; j < top; ++j) {
-      chosen_z[j] = expf(chosen_z[j] - mx);
-      sum += chosen_z[j];
-    }
-    for (int j = 0; j < top; ++j) {
-      ids[(size_t)row * top + j] = chosen_e[j];
-      wts[(size_t)row * top + j] = chosen_z[j] / sum;
-    }
+    for (int j = 0; j < top; ++j) sum += __shfl_sync(0xffffffffu, score, j);
+    weight = score / (sum + 1e-20f);
+  } else {
+    float mx = __shfl_sync(0xffffffffu, own_z, 0), sum = 0.f;
+    for (int j = 1; j < top; ++j) mx = fmaxf(mx, __shfl_sync(0xffffffffu, own_z, j));
+    const float e = mine ? expf(own_z - mx) : 0.f;
+    for (int j = 0; j < top; ++j) sum += __shfl_sync(0xffffffffu, e, j);
+    weight = e / sum;
   }
+  if (mine) ids[at] = own_e, wts[at] = weight;
 }
 
 // A block takes kRows rows, a warp kExperts experts at a time for all of them, and then chooses for row after row. Few rows:
 // 1 x 1, so that a row's 16-byte loads are all in flight (a warp per four experts took 14.5 us for 4 rows of width 2,048 and
-// 16 experts, this 7.3 us); many: 4 x 4, sixteen dot products for every eight loads (6,300 rows 39 us; one row a block took
+// 16 experts, this 7.3 us), and the weights and corrections, which no kernel of a step writes, ahead of the wait (4 rows
+// in a decode step 8.7 us before, with the choices in local memory, 8.2 now; Luzitar's pass 17.56 -> 17.34 ms); many: 4 x 4, sixteen dot products for every eight loads (6,300 rows 39 us; one row a block took
 // 51 us, 4 x 1 69 us).
-template <typename T, int kRows, int kExperts>
-__global__ void __launch_bounds__(kRows > 1 ? 512 : 1024) moe_router_kernel(const T* __restrict__ x, long long ldx, const void* __restrict__ w, int w_dtype,
+// kHold: 1 x 1 with no more experts than the block has warps and no more of a row than a lane holds.
+constexpr int kHoldPieces = 8, kHoldExperts = 24, kCorrCopy = 512;
+template <typename T, int kRows, int kExperts, bool kHold>
+__global__ void __launch_bounds__(kHold ? 32 * kHoldExperts : (kRows > 1 ? 512 : 1024)) moe_router_kernel(const T* x, long long ldx, const void* __restrict__ w, int w_dtype,
                                                           int rows, int K, int E, int top, int* __restrict__ ids, float* __restrict__ wts,
                                                           int scoring, const float* __restrict__ correction, int n_groups, int keep_groups,
                                                           float weight_scale) {
-  pdl_start();
-  // per row: logits [E], scores [E], group scores [E]; then, per row, which experts are taken [E bytes]
-  extern __shared__ float smem[];
+  pdl_trigger();
+  // the corrections [E] (up to kCorrCopy); per row: logits [E], scores [E], group scores [E]; then, per row, which experts are taken [E bytes]
+  extern __shared__ float router_smem[];
+  const float* const corr = correction && E <= kCorrCopy ? router_smem : correction;
+  float* const smem = router_smem + (E <= kCorrCopy ? E : 0);
+  if (correction && E <= kCorrCopy)
+    for (int e = threadIdx.x; e < E; e += blockDim.x) router_smem[e] = correction[e];
   const int warps = blockDim.x >> 5, wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * kRows;
   constexpr int kVec = 16 / (int)sizeof(T);
   const bool vec = w_dtype == (sizeof(T) == 2 ? OI_BF16 : OI_F32) && K % kVec == 0 && ldx % kVec == 0 && (uintptr_t)x % 16 == 0 &&
                    (uintptr_t)w % 16 == 0;
+  uint4 wh[kHold ? kHoldPieces : 1];
+  if constexpr (kHold) {
+#pragma unroll
+    for (int t = 0; t < kHoldPieces; ++t)
+      if (wi < E && (t * 32 + lane) * kVec < K) wh[t] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(w) + (size_t)wi * K) + t * 32 + lane);
+  }
+  pdl_wait();
   const T* xr[kRows];        // rows beyond the last read that one again and are not stored
 #pragma unroll
   for (int r = 0; r < kRows; ++r) xr[r] = x + (size_t)min(row0 + r, rows - 1) * ldx;
   for (int e0 = wi * kExperts; e0 < E; e0 += warps * kExperts) {
     float acc[kRows][kExperts] = {};
-    if (vec) {               // a lane takes 16 bytes of the rows and of the experts' weights at a time
+    if constexpr (kHold) {
+      uint4 xh[kHoldPieces];
+#pragma unroll
+      for (int t = 0; t < kHoldPieces; ++t)
+        if ((t * 32 + lane) * kVec < K) xh[t] = *(reinterpret_cast<const uint4*>(xr[0]) + t * 32 + lane);
+#pragma unroll
+      for (int t = 0; t < kHoldPieces; ++t)
+        if ((t * 32 + lane) * kVec < K) {
+#pragma unroll
+          for (int i = 0; i < kVec; ++i) acc[0][0] += to_f32(reinterpret_cast<const T*>(&wh[t])[i]) * to_f32(reinterpret_cast<const T*>(&xh[t])[i]);
+        }
+    } else if (vec) {        // a lane takes 16 bytes of the rows and of the experts' weights at a time
       const T* wrow[kExperts];      // experts beyond the last read that one again and are not stored
 #pragma unroll
       for (int q = 0; q < kExperts; ++q) wrow[q] = reinterpret_cast<const T*>(w) + (size_t)min(e0 + q, E - 1) * K;
@@ -207,7 +225,7 @@ __global__ void __launch_bounds__(kRows > 1 ? 512 : 1024) moe_router_kernel(cons
   __syncthreads();
   for (int r = wi; r < kRows && row0 + r < rows; r += warps)
     choose(smem + (size_t)r * 3 * E, reinterpret_cast<unsigned char*>(smem + (size_t)kRows * 3 * E) + (size_t)r * E, row0 + r, E, top, ids, wts,
-           scoring, correction, n_groups, keep_groups, weight_scale);
+           scoring, corr, n_groups, keep_groups, weight_scale);
 }
 // One block per expert e. sorted[first_e + i] = the i-th pair (in ascending pair number) that chose e; tiles of tile_m
 // sorted places that belong to one expert: tile_info[3 * t] = expert, first place, rows. tile_info's last word
@@ -1003,15 +1021,19 @@ OI_API int oi_moe_route_scored(const void* x, int dtype, long long ldx, const vo
   constexpr int kMany = 4;
   const bool many = rows >= 8 * 148 && all <= 512;
   const int per_block = many ? kMany : 1, blocks = (rows + per_block - 1) / per_block;
-  const size_t smem = per_block * (3 * (size_t)all * sizeof(float) + (size_t)all) + 16;
+  const size_t smem = (all <= kCorrCopy ? (size_t)all * sizeof(float) : 0) + per_block * (3 * (size_t)all * sizeof(float) + (size_t)all) + 16;
   const int groups_of = many ? (all + 3) / 4 : all, threads = 32 * (groups_of > (many ? 16 : 32) ? (many ? 16 : 32) : groups_of);
-#define OI_ROUTER(T, ROWS)                                                                                                          \
-  oi_launch(moe_router_kernel<T, ROWS, ROWS>, blocks, threads, smem, s, (const T*)x, ldx, w_router, w_dtype, rows, K, all, top, ids, wts, \
+  auto hold = [&](int esize) {
+    return !many && all <= kHoldExperts && w_dtype == dtype && K * esize % 16 == 0 && K * esize <= 16 * 32 * kHoldPieces && ldx * esize % 16 == 0 &&
+           (uintptr_t)x % 16 == 0 && (uintptr_t)w_router % 16 == 0;
+  };
+#define OI_ROUTER(T, ROWS, HOLD)                                                                                                    \
+  oi_launch(moe_router_kernel<T, ROWS, ROWS, HOLD>, blocks, threads, smem, s, (const T*)x, ldx, w_router, w_dtype, rows, K, all, top, ids, wts, \
             scoring, correction, n_groups, keep_groups, weight_scale)
   if (dtype == OI_F32) {
-    if (many) OI_ROUTER(float, kMany); else OI_ROUTER(float, 1);
+    if (many) OI_ROUTER(float, kMany, false); else if (hold(4)) OI_ROUTER(float, 1, true); else OI_ROUTER(float, 1, false);
   } else if (dtype == OI_BF16) {
-    if (many) OI_ROUTER(bf16, kMany); else OI_ROUTER(bf16, 1);
+    if (many) OI_ROUTER(bf16, kMany, false); else if (hold(2)) OI_ROUTER(bf16, 1, true); else OI_ROUTER(bf16, 1, false);
   } else {
     OI_REQUIRE(false, "moe_route: unknown dtype code %d", dtype);
   }
