@@ -371,7 +371,12 @@ class Model:
         h, branch, u = buf(H, f32), buf(H, f32), buf(H)
         low = buf(H) if dt != f32 else None
         hist = torch.empty((len(self.calls) + 1, T, H), dtype=f32, device=dev) if desc.averaged else None
-        ahead = torch.empty((native.DEPTH_AHEAD, T, H), dtype=f32, device=dev) if desc.averaged and len(self.calls) > 4 else None
+        ahead = None
+        if desc.averaged and len(self.calls) > 4:
+            try:
+                ahead = torch.empty((native.DEPTH_AHEAD, T, H), dtype=f32, device=dev)
+            except torch.cuda.OutOfMemoryError:      # a step that fits without: every average reads the whole history
+                pass
         proj, mixed, z = buf(desc.max_in), buf(desc.max_mixed), buf(desc.max_inter)
         steps = (native.AttnStep * len(keys))()
         kept = []

@@ -1898,3 +1898,34 @@ def test_depth_averages_share_their_earlier_terms(rows, hidden, coef_dtype):
         hs.append(h)
         lows.append(low)
     assert torch.equal(*hists) and torch.equal(*hs) and torch.equal(*lows)
+
+
+def test_steps_with_score_routers_keep_the_streaming_product():
+    """Inside ``policy.streamed_products`` this thread's products (another thread's are not meant) are the streaming kernel's bit for
+    bit, and outside the few-rows kernel's."""
+    import threading
+
+    from openinfer_b200.kernels import lib as klib
+    from openinfer_b200.kernels import linear as lin
+    from openinfer_b200.kernels import policy
+    L = klib.load()
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x = torch.randn(4, 2048, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(1024, 2048, device=DEV, generator=g) * 2048 ** -0.5).to(torch.bfloat16)
+    stream = torch.cuda.current_stream().cuda_stream
+    few, streamed = (torch.empty(4, 1024, device=DEV) for _ in range(2))
+    klib.check(L.oi_gemm_few(few.data_ptr(), 0, 1024, x.data_ptr(), 2048, w.data_ptr(), 2048, 4, 1024, 2048, 0, 0, 0.0, 0.0, stream), "few")
+    klib.check(L.oi_gemm_stream(streamed.data_ptr(), 0, 1024, x.data_ptr(), 2048, w.data_ptr(), 2048, 4, 1024, 2048,
+                                L.oi_stream_slices(1024, 2048), 0, stream), "stream")
+    assert not torch.equal(few, streamed)
+    other = []
+    with pytest.raises(ValueError):
+        with policy.streamed_products():
+            assert torch.equal(lin.linear(x, w, out_dtype=torch.float32), streamed)
+            t = threading.Thread(target=lambda: other.append(lin.linear(x, w, out_dtype=torch.float32)))
+            t.start()
+            t.join()
+            raise ValueError
+    torch.cuda.synchronize()
+    assert torch.equal(other[0], few)
+    assert torch.equal(lin.linear(x, w, out_dtype=torch.float32), few)
