@@ -386,6 +386,22 @@ OI_API int oi_forward(const OiModelDesc* m, const OiStepDesc* st, void* stream) 
   return OI_OK;
 }
 
+// The averages behind layer `layer` (whose own has `results` earlier terms) that its launch may add up terms for. Only those whose
+// coefficients are as many as their turn asks for: the kernel reads `results` + 1 of each. One that is not so, and what lies
+// behind it, is left out here and refused by oi_forward_branch when its turn comes.
+OI_API int oi_depth_ahead_layers(const OiBranchLayerDesc* layers, int num_layers, int layer, int results, OiDepthAhead* ahead) {
+  OI_REQUIRE(layers && ahead && layer >= 0 && layer < num_layers && results >= 0, "depth_ahead_layers: layer %d of %d", layer, num_layers);
+  ahead->next = 0;
+  int terms = results + 2;
+  for (int q = layer + 1; q < num_layers && ahead->next < kDepthAhead; ++q) {
+    if (!layers[q].depth_coef) continue;
+    if (layers[q].depth_terms != terms++) break;
+    ahead->coef[ahead->next] = layers[q].depth_coef;
+    ahead->coef_dtype[ahead->next++] = layers[q].depth_dtype;
+  }
+  return OI_OK;
+}
+
 OI_API int oi_forward_branch(const OiBranchModelDesc* m, const OiBranchStepDesc* st, void* stream) {
   OI_REQUIRE(m && st && m->layers && (st->num_attn_steps == 0 || st->attn_steps), "forward_branch: null description");
   const int T = st->tokens, H = m->hidden, dt = m->dtype;
@@ -413,8 +429,7 @@ OI_API int oi_forward_branch(const OiBranchModelDesc* m, const OiBranchStepDesc*
         d.sum = st->ahead + left * hist_stride;
         d.from = ahead_from;
       } else if (results >= 4) {
-        for (int q = i + 1; q < m->num_layers && d.next < kDepthAhead; ++q)
-          if (m->layers[q].depth_coef) d.coef[d.next] = m->layers[q].depth_coef, d.coef_dtype[d.next++] = m->layers[q].depth_dtype;
+        OI_TRY(oi_depth_ahead_layers(m->layers, m->num_layers, i, results, &d));
         d.out = st->ahead;
         d.stride = hist_stride;
         ahead_from = results, ahead_used = 0, ahead_have = d.next;

@@ -561,3 +561,5 @@ typedef struct OiBranchStepDesc {
 } OiBranchStepDesc;
 
 OI_API int oi_forward_branch(const OiBranchModelDesc* model, const OiBranchStepDesc* step, void* stream);
+// Which averages behind layer `layer` its launch adds up terms for: coef, coef_dtype and next of `ahead` (no GPU is used).
+OI_API int oi_depth_ahead_layers(const OiBranchLayerDesc* layers, int num_layers, int layer, int results, OiDepthAhead* ahead);

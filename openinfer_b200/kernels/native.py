@@ -156,6 +156,7 @@ def declare(lib) -> None:
     lib.oi_forward.argtypes, lib.oi_forward.restype = [POINTER(ModelDesc), POINTER(StepDesc), P], c_int
     lib.oi_dense_mlp.argtypes, lib.oi_dense_mlp.restype = [P, P, I, I, I, I, P, I, P, I, P, I, c_float, c_float, P, P], c_int
     lib.oi_forward_branch.argtypes, lib.oi_forward_branch.restype = [POINTER(BranchModelDesc), POINTER(BranchStepDesc), P], c_int
+    lib.oi_depth_ahead_layers.argtypes, lib.oi_depth_ahead_layers.restype = [POINTER(BranchLayerDesc), I, I, I, POINTER(DepthAhead)], c_int
     lib.oi_launches.argtypes, lib.oi_launches.restype = [], ctypes.c_ulonglong
     lib.oi_launch_fence.argtypes, lib.oi_launch_fence.restype = [], c_int
     lib.oi_branch_norm_add_ahead.argtypes = [P, P, I, P, I, I, I, c_float, c_float, P, L, I, P, I, P, POINTER(DepthAhead), P]

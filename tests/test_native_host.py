@@ -1,0 +1,32 @@
+"""What the native library decides on the host, called without a GPU."""
+import ctypes
+
+import pytest
+
+from openinfer_b200.kernels import lib as klib
+from openinfer_b200.kernels import native
+
+
+def _averages_behind(terms, layer, results):
+    """Indexes of the layers whose averages layer ``layer`` adds up terms for; ``terms``: what each layer averages (None: nothing)."""
+    layers = (native.BranchLayerDesc * len(terms))()
+    for i, t in enumerate(terms):
+        if t is not None:
+            layers[i].depth_coef, layers[i].depth_terms, layers[i].depth_dtype = 1000 + i, t, i % 2
+    d = native.DepthAhead()
+    assert klib.load().oi_depth_ahead_layers(layers, len(terms), layer, results, ctypes.byref(d)) == 0
+    chosen = [d.coef[q] - 1000 for q in range(d.next)]
+    assert [d.coef_dtype[q] for q in range(d.next)] == [i % 2 for i in chosen]
+    return chosen
+
+
+@pytest.mark.parametrize("terms,layer,results,want", [
+    (list(range(2, 12)), 3, 4, [4, 5, 6]),
+    (list(range(2, 12)), 7, 8, [8, 9]),                                # fewer than three layers left
+    (list(range(2, 12)), 9, 10, []),
+    ([2, 3, None, 4, 5, None, 6, None, 7, 8], 4, 4, [6, 8, 9]),        # layers in between that average nothing
+    ([2, 3, 4, 5, 6, 3, 8, 9, 10, 11], 3, 4, [4]),                     # coefficients fewer than their turn asks for: not read
+    ([2, 3, 4, 5, 5, 7, 8, 9, 10, 11], 3, 4, []),
+])
+def test_sums_ahead_are_of_averages_whose_coefficients_are_all_there(terms, layer, results, want):
+    assert _averages_behind(terms, layer, results) == want
