@@ -107,7 +107,8 @@ class SlotClearer:
     def clear(self, slot: int) -> None:
         if not 0 <= slot < self.slots:
             raise KernelError(f"clear_slots: slot {slot} of {self.slots}")
-        _lib.check(_lib.load().oi_clear_slots(self.table.data_ptr(), len(self.tensors), self.max_bytes, slot, _stream()), "clear_slots")
+        with torch.cuda.device(self.table.device):       # whatever device is the calling thread's own, as a fill of the tensors would
+            _lib.check(_lib.load().oi_clear_slots(self.table.data_ptr(), len(self.tensors), self.max_bytes, slot, _stream()), "clear_slots")
 
 
 class UploadRing:

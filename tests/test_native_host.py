@@ -30,3 +30,35 @@ def _averages_behind(terms, layer, results):
 ])
 def test_sums_ahead_are_of_averages_whose_coefficients_are_all_there(terms, layer, results, want):
     assert _averages_behind(terms, layer, results) == want
+
+
+def test_slots_are_cleared_on_the_tensors_own_device(monkeypatch):
+    """The calling thread's current device may be another than the cache's."""
+    import torch
+
+    from openinfer_b200.kernels import ops
+    current, launched = ["another device"], []
+
+    class Device:
+        def __init__(self, device):
+            self.device = device
+
+        def __enter__(self):
+            self.was, current[0] = current[0], self.device
+
+        def __exit__(self, *exc):
+            current[0] = self.was
+
+    class Library:
+        @staticmethod
+        def oi_clear_slots(table, tensors, max_bytes, slot, stream):
+            launched.append((current[0], stream, slot, tensors, max_bytes))
+            return 0
+
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    monkeypatch.setattr(ops, "_cuda", lambda *tensors: None)
+    monkeypatch.setattr(ops, "_stream", lambda: f"stream of {current[0]}")
+    monkeypatch.setattr(ops._lib, "load", lambda: Library)
+    ops.SlotClearer([torch.ones(4, 3), torch.ones(4, 2, 8)]).clear(2)
+    assert launched == [(torch.device("cpu"), "stream of cpu", 2, 2, 64)]
+    assert current[0] == "another device"
