@@ -23,12 +23,14 @@ static int g_pdl = 1;
 int oi_pdl_enabled() { return g_pdl; }
 // A kernel whose writes later kernels read BEFORE their own wait (the step's metadata) asks for the next launch to be
 // an ordinary one: that kernel then starts after the writer has completed, and the chain behind it after that.
-static int g_fence_next = 0;
+// The next launch of the host thread that asked: another thread's launch in between (a request opened beside a step) leaves it.
+static thread_local int g_fence_next = 0;
 void oi_fence_next_launch() { g_fence_next = 1; }
 OI_API int oi_launch_fence() {
   g_fence_next = 1;
   return OI_OK;
 }
+OI_API int oi_launch_fence_pending() { return g_fence_next; }
 int oi_take_launch_fence() {
   const int v = g_fence_next;
   g_fence_next = 0;

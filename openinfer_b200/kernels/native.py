@@ -159,6 +159,7 @@ def declare(lib) -> None:
     lib.oi_depth_ahead_layers.argtypes, lib.oi_depth_ahead_layers.restype = [POINTER(BranchLayerDesc), I, I, I, POINTER(DepthAhead)], c_int
     lib.oi_launches.argtypes, lib.oi_launches.restype = [], ctypes.c_ulonglong
     lib.oi_launch_fence.argtypes, lib.oi_launch_fence.restype = [], c_int
+    lib.oi_launch_fence_pending.argtypes, lib.oi_launch_fence_pending.restype = [], c_int
     lib.oi_branch_norm_add_ahead.argtypes = [P, P, I, P, I, I, I, c_float, c_float, P, L, I, P, I, P, POINTER(DepthAhead), P]
     lib.oi_branch_norm_add_ahead.restype = c_int
     lib.oi_gemm_stream_fused.argtypes = [P, I, L, P, L, P, L, I, I, I, I, I, POINTER(StreamEpilogue), P]

@@ -1,5 +1,6 @@
 """What the native library decides on the host, called without a GPU."""
 import ctypes
+import threading
 
 import pytest
 
@@ -62,3 +63,25 @@ def test_slots_are_cleared_on_the_tensors_own_device(monkeypatch):
     ops.SlotClearer([torch.ones(4, 3), torch.ones(4, 2, 8)]).clear(2)
     assert launched == [(torch.device("cpu"), "stream of cpu", 2, 2, 64)]
     assert current[0] == "another device"
+
+
+def test_a_launch_fence_belongs_to_the_thread_that_asked_for_it():
+    """Between a step's metadata and its first kernel another thread may launch (it opens a request): that launch does not use up the
+    plain order which the step's first kernel was to get."""
+    L = klib.load()
+    seen = []
+
+    def other():
+        seen.append(L.oi_launch_fence_pending())
+
+    def asks():
+        L.oi_launch_fence()
+        t = threading.Thread(target=other)
+        t.start()
+        t.join()
+        seen.append(L.oi_launch_fence_pending())
+
+    t = threading.Thread(target=asks)       # a thread of its own: this test's fence reaches no launch
+    t.start()
+    t.join()
+    assert seen == [0, 1]
