@@ -85,10 +85,21 @@ def gate_up_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, act: str = "silu"
 
 
 def stream_status() -> int:
-    """0, or which bounded wait of the streaming kernel ran out since the last call (synchronises)."""
+    """0, or which bounded wait of a decode product ran out since the last call (synchronises): the streaming kernel's code, or
+    100 more than that of the product of few rows."""
+    few = few_status()
+    return _status("oi_gemm_stream_status") or (100 + few if few else 0)
+
+
+def few_status() -> int:
+    """The same of the product of few rows alone."""
+    return _status("oi_gemm_few_status")
+
+
+def _status(entry: str) -> int:
     from ctypes import byref, c_int
     v = c_int(0)
-    _lib.check(_lib.load().oi_gemm_stream_status(byref(v)), "gemm_stream_status")
+    _lib.check(getattr(_lib.load(), entry)(byref(v)), entry)
     return v.value
 
 

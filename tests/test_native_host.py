@@ -85,3 +85,19 @@ def test_a_launch_fence_belongs_to_the_thread_that_asked_for_it():
     t.start()
     t.join()
     assert seen == [0, 1]
+
+
+@pytest.mark.parametrize("stream,few,want", [(0, 0, 0), (2, 0, 2), (0, 1, 101), (3, 2, 3)])
+def test_the_decode_products_status_is_both_kernels(monkeypatch, stream, few, want):
+    """Which of the two kernels took a product is the dispatch's affair: one question covers both."""
+    from openinfer_b200.kernels import linear
+
+    def entry(code):
+        def fn(v):
+            v._obj.value = code
+            return 0
+        return staticmethod(fn)
+
+    library = type("Library", (), {"oi_gemm_stream_status": entry(stream), "oi_gemm_few_status": entry(few)})
+    monkeypatch.setattr(linear._lib, "load", lambda: library)
+    assert linear.stream_status() == want and linear.few_status() == few
