@@ -371,12 +371,6 @@ class Model:
         h, branch, u = buf(H, f32), buf(H, f32), buf(H)
         low = buf(H) if dt != f32 else None
         hist = torch.empty((len(self.calls) + 1, T, H), dtype=f32, device=dev) if desc.averaged else None
-        ahead = None
-        if desc.averaged and len(self.calls) > 4:
-            try:
-                ahead = torch.empty((native.DEPTH_AHEAD, T, H), dtype=f32, device=dev)
-            except torch.cuda.OutOfMemoryError:      # a step that fits without: every average reads the whole history
-                pass
         proj, mixed, z = buf(desc.max_in), buf(desc.max_mixed), buf(desc.max_inter)
         steps = (native.AttnStep * len(keys))()
         kept = []
@@ -393,6 +387,12 @@ class Model:
         n_want = 0 if row_idx is None else row_idx.numel()
         wanted = buf(H, rows=n_want) if n_want else None
         logits = buf(self.spec.vocab_size, dtype=f32, rows=n_want) if n_want else None
+        ahead = None
+        if desc.averaged and len(self.calls) > 4:    # behind everything that the step cannot do without
+            try:
+                ahead = torch.empty((native.DEPTH_AHEAD, T, H), dtype=f32, device=dev)
+            except torch.cuda.OutOfMemoryError:      # a step that fits without: every average reads the whole history
+                pass
 
         def ptr(t):
             return 0 if t is None else t.data_ptr()

@@ -89,6 +89,13 @@ CASE_H = {
     "norm": {"eps": 1e-6}, "canon": {"taps": 3},
     "layers": [_layer(2, 8, 8, 320, 1.2, window=30, ff=32), _layer(3, 8, 8, 320, 0.9, window=12, kv_from=0)],
 }
+# thirteen layers: three times over, a layer adds up what later averages need of the history (behind the last one a single layer is left)
+CASE_DEEP = {
+    "architecture": "Delunex", "vocab": 119, "width": 64, "logit_scale": 0.8, "embedding": {"scale": 3.0},
+    "norm": {"eps": 1e-6}, "canon": {"taps": 3},
+    "layers": [_layer(2 + i % 2, 16, 8 + 8 * (i % 2), 32, 0.8, window=(21, None, 34)[i % 3], kv_from=i - i % 3 if i % 3 else None,
+                      ff=None if i in (3, 5, 11) else 40 + 8 * i) for i in range(13)],
+}
 CASES = {"A": (CASE_A, 11), "B": (CASE_B, 12), "C": (CASE_C, 13), "D": (CASE_D, 14), "E": (CASE_E, 15), "F": (CASE_F, 16),
          "G": (CASE_G, 17), "H": (CASE_H, 18)}
 

@@ -12,7 +12,7 @@ import pytest
 import torch
 
 import plain_delunex as plain
-from delunex_cases import CASES, assert_logits, make_folder, oracle, read_folder, tokens_for
+from delunex_cases import CASE_DEEP, CASES, assert_logits, make_folder, oracle, read_folder, tokens_for
 from helpers import (ROOT, count_page_handouts, replay_in_process, replay_trace_run, round64, trace_mixed, trace_portions,
                      trace_tail, trace_whole)
 
@@ -371,6 +371,46 @@ def test_native_step_and_part_by_part_step_give_the_same_bits(folders, name, dty
         assert (runner.model._native is not None) == (native and not (dtype == "bfloat16" and "canon" not in cfg))
     for rid in requests:
         assert torch.equal(out[0][rid], out[1][rid]), f"{name}/{dtype}/{rid}"
+
+
+@pytest.fixture(scope="module")
+def deep(tmp_path_factory):
+    return make_folder(str(tmp_path_factory.mktemp("dlxdeep")), CASE_DEEP, 19)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("allocate", ["all", "mandatory only", "nothing behind the sums ahead"])
+def test_a_step_needs_no_room_for_sums_ahead(deep, dtype, allocate, monkeypatch):
+    """The buffer that averages leave sums in is asked for behind all that the step cannot do without, and a step that
+    does not get it gives the same bits."""
+    from openinfer_b200.engine.runner import StepEntry
+    from openinfer_b200.kernels import native
+    tokens = tokens_for(CASE_DEEP, 50, 3)
+    shape = (native.DEPTH_AHEAD, len(tokens), CASE_DEEP["width"])
+    empty, asked = torch.empty, []
+
+    def limited(*size, **kw):
+        t = tuple(size[0]) if len(size) == 1 and not isinstance(size[0], int) else size
+        if (t == shape and allocate == "mandatory only") or (asked and allocate == "nothing behind the sums ahead"):
+            asked.append(t)
+            raise torch.cuda.OutOfMemoryError("no room (a test)")
+        if t == shape:
+            asked.append(t)
+        return empty(*size, **kw)
+
+    runner = runner_for(deep, dtype, graphs=False)
+    want = runner.step([StepEntry("a", tokens, list(range(len(tokens))))]).clone()
+    run = runner.model._run_native_branch
+
+    def run_limited(*args):
+        with monkeypatch.context() as m:
+            m.setattr(torch, "empty", limited)
+            return run(*args)
+
+    monkeypatch.setattr(runner.model, "_run_native_branch", run_limited)
+    got = runner.step([StepEntry("b", tokens, list(range(len(tokens))))])
+    assert asked and asked[0] == shape
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("rows", [1, 8, 32, 33, 100, 300, 2100])
