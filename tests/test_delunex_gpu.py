@@ -379,6 +379,25 @@ def deep(tmp_path_factory):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+def test_sums_ahead_in_whole_models(deep, dtype):
+    """Averages that start from what an earlier layer left (the native step) and averages that read the whole history (part by
+    part): the same bits in portions, mixed steps and recorded single-token steps, with layers without a feed-forward among the
+    thirteen; in float32 also the oracle's logits."""
+    requests = {f"d{i}": tokens_for(CASE_DEEP, n, 80 + i) for i, n in enumerate([70, 9, 41])}
+    steps = trace_mixed(requests, 512, seed=2, max_live=3, tail=12)
+    out = []
+    for native in (True, False):
+        runner = runner_for(deep, dtype, max_tokens=512)
+        runner.model.native_step = native
+        out.append(replay_in_process(runner, steps))
+        assert (runner.model._native is not None) == native
+    for rid, toks in requests.items():
+        assert torch.equal(out[0][rid], out[1][rid]), f"{dtype}/{rid}"
+        if dtype == "float32":
+            assert_logits(out[0][rid], oracle(deep, toks), dtype, rid)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("allocate", ["all", "mandatory only", "nothing behind the sums ahead"])
 def test_a_step_needs_no_room_for_sums_ahead(deep, dtype, allocate, monkeypatch):
     """The buffer that averages leave sums in is asked for behind all that the step cannot do without, and a step that

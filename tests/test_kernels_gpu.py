@@ -1777,24 +1777,27 @@ def test_embedding_widened(hidden):
 # the ring holds at once (12,288 x 2,048 and 2,048 x 6,144); every number of tokens' tiles
 @pytest.mark.parametrize("M,N,K", [(1, 5, 64), (2, 13, 192), (8, 1024, 1024), (9, 1000, 1088), (16, 300, 3072), (3, 2376, 2112),
                                    (8, 12288, 2048), (7, 2048, 6144), (16, 16384, 1024), (12, 4104, 4096)])
-@pytest.mark.parametrize("act", ["none", "xielu", "silu", "swiglu_clamp"])
+@pytest.mark.parametrize("act", ["none", "xielu", "silu", "gelu_tanh", "swiglu_clamp"])
 def test_gemm_few(M, N, K, act):
     """The product of few rows against float64, into rows with a gap behind them; its results do not depend on the other rows."""
     from openinfer_b200.kernels import lib as klib
     L = klib.load()
-    glu = act in ("silu", "swiglu_clamp")
+    glu = act in ("silu", "gelu_tanh", "swiglu_clamp")
     N = -(-N // 128) * 128 if glu else N
     g = torch.Generator(device=DEV).manual_seed(N + K + M)
     x = torch.randn(M, K + 16, device=DEV, generator=g).to(torch.bfloat16)[:, :K]
     w = (torch.randn(N, K + 8, device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)[:, :K]
     ref = x.double() @ w.double().t()
-    code, p0, p1 = {"none": (0, 0.0, 0.0), "xielu": (3, 0.8, 0.9), "silu": (1, 0.0, 0.0), "swiglu_clamp": (4, 0.5, 0.0)}[act]
+    code, p0, p1 = {"none": (0, 0.0, 0.0), "xielu": (3, 0.8, 0.9), "silu": (1, 0.0, 0.0), "gelu_tanh": (2, 0.0, 0.0),
+                    "swiglu_clamp": (4, 0.5, 0.0)}[act]
     if act == "xielu":
         ref = torch.where(ref > 0, p0 * ref * ref, p1 * (torch.expm1(ref) - ref)) + 0.5 * ref
     if glu:
         a, b = ref.view(M, N // 128, 2, 64).unbind(2)
         if act == "silu":
             ref = a * torch.sigmoid(a) * b
+        elif act == "gelu_tanh":
+            ref = 0.5 * a * (1.0 + torch.tanh(math.sqrt(2.0 / math.pi) * (a + 0.044715 * a ** 3))) * b
         else:
             a, b = a.clamp(max=p0), b.clamp(-p0, p0)
             ref = a * torch.sigmoid(1.702 * a) * (b + 1.0)
@@ -1898,6 +1901,31 @@ def test_depth_averages_share_their_earlier_terms(rows, hidden, coef_dtype):
         hs.append(h)
         lows.append(low)
     assert torch.equal(*hists) and torch.equal(*hs) and torch.equal(*lows)
+
+
+@pytest.mark.parametrize("M,N,K,x_off,few", [
+    (4, 1024, 1024, 0, True), (16, 2368, 4096, 0, True), (8, 2368, 6144, 0, True), (16, 96, 64, 0, True),
+    (4, 1024, 1024, 8, False),                                        # rows of x 16 bytes off
+    (4, 96, 1000, 0, False), (17, 1024, 1024, 0, False),              # K no multiple of 64; one row too many
+    (16, 1024, 6144, 0, False), (8, 2376, 4096, 0, False)])           # x's rows do not fit; longer rows than 148 CTAs take at a time
+def test_which_kernel_takes_a_decode_product(M, N, K, x_off, few):
+    """The dispatch's results are those of the kernel that the rule names, bit for bit."""
+    from openinfer_b200.kernels import lib as klib
+    from openinfer_b200.kernels import linear as lin
+    L = klib.load()
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x = torch.randn(M * K + 8, device=DEV, generator=g).to(torch.bfloat16)[x_off: x_off + M * K].view(M, K)
+    w = (torch.randn(N, K, device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)
+    want = torch.empty(M, N, device=DEV)
+    args = (want.data_ptr(), 0, N, x.data_ptr(), K, w.data_ptr(), K, M, N, K)
+    stream = torch.cuda.current_stream().cuda_stream
+    if few:
+        klib.check(L.oi_gemm_few(*args, 0, 0, 0.0, 0.0, stream), "gemm_few")
+    else:
+        klib.check(L.oi_gemm_stream(*args, L.oi_stream_slices(N, K), 0, stream), "gemm_stream")
+    got = lin.linear(x, w, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and lin.stream_status() == 0
 
 
 def test_steps_with_score_routers_keep_the_streaming_product():

@@ -101,3 +101,33 @@ def test_the_decode_products_status_is_both_kernels(monkeypatch, stream, few, wa
     library = type("Library", (), {"oi_gemm_stream_status": entry(stream), "oi_gemm_few_status": entry(few)})
     monkeypatch.setattr(linear._lib, "load", lambda: library)
     assert linear.stream_status() == want and linear.few_status() == few
+
+
+@pytest.mark.parametrize("design,name,streamed", [("rolevik", "A", True), ("luzitar", "A", True), ("bubalix", "A", False), ("delunex", "A", False)])
+def test_steps_whose_experts_are_chosen_by_scores_run_with_streamed_products(monkeypatch, design, name, streamed):
+    """Router scores: layers and head run under ``policy.streamed_products``, in that thread and for that long; a table of experts or
+    no experts: they do not."""
+    import importlib
+
+    import torch
+
+    from openinfer_b200.config.base import resolve_architecture
+    from openinfer_b200.parts.model import Model
+    raw = importlib.import_module(f"{design}_cases").CASES[name][0]
+    entry = resolve_architecture(raw)
+    model = Model(entry.build_spec(entry.config_cls.from_dict(raw)), torch.bfloat16)
+    L = klib.load()
+    seen = []
+
+    def now(*_):
+        was = L.oi_streamed_products(0)
+        L.oi_streamed_products(was)
+        seen.append(bool(was))
+        return None, None
+
+    model.native_step = False
+    monkeypatch.setattr(model, "forward", now)
+    monkeypatch.setattr(model, "logits", now)
+    model.run(None, torch.zeros(1))
+    now()
+    assert model.routes_by_score == streamed and seen == [streamed, streamed, False]
