@@ -34,16 +34,22 @@ bool tma_ok(const void* x, long long ldx, const void* w, long long ldw, int K) {
 thread_local int t_streamed = 0;
 
 // How many K slices (CTAs per cluster) the streaming kernel uses: one when the tiles of 128 weight rows alone
-// fill the GPU, else the fewest slices that give every SM a CTA, each slice at least two k blocks long, while the CTAs are
-// no more than 256: two fit on an SM, but clusters of 4 or 8 do not find room on all of them at once.
+// fill the GPU, else the fewest slices that give every SM a CTA, each slice at least two k blocks long, while all CTAs run at
+// once: two fit on an SM, but clusters of 8 only 33 at a time (264 CTAs), of 4 only 70 (280), and what is left over runs alone.
 // Measured on B200 at M = 8 (us, inside a CUDA graph): N 6144 K 4096: 14.2 with 4 slices (16.1 with 2, 17.0
 // with 8); N 4096 K 4096: 11.1 with 8 (11.8 with 4); N 4096 K 12288: 20.9 with 8 (22.1 with 4); N 24576 and
-// N 151936: one slice (34.4 and 188). With the norm kernel before it: N 4608 K 2048: 7.6 with 4 slices (10.2 with 8, 288
-// CTAs); N 9216 K 2048: 11.5 with 2 (14.3 with 4, 288 CTAs).
+// N 151936: one slice (34.4 and 188). With the norm kernel before it, at M = 1: N 4224 K 4096: 8.4 with 8 slices (264 CTAs; 9.7
+// with 4), N 4352 9.8 with 4 (12.7 with 8, 272 CTAs); N 8960 K 4096: 14.4 with 4 (280 CTAs; 15.5 with 2), N 9216 15.7 with 2 (21.1
+// with 4, 288 CTAs). Clusters of 2 all fit, but more than 256 CTAs of short slices do not pay for their sums: N 16512 at 32 rows
+// K 2048 16.9 with one slice (17.8 with 2), K 3072 22.7 with 2 (23.6 with one), K 8192 49.9 (54.3).
 int stream_slices(int N, int K) {
   const int tiles = (N + 127) / 128, num_kb = (K + 63) / 64;
+  auto at_once = [&](int slices) {
+    const int ctas = tiles * slices;
+    return slices == 8 ? ctas <= 264 : (slices == 4 ? ctas <= 280 : ctas <= 256 || num_kb >= 48);
+  };
   int c = 1;
-  while (c < 8 && tiles * c < sm_count() && (tiles * 2 * c <= 256 || t_streamed) && num_kb / (2 * c) >= 2) c *= 2;
+  while (c < 8 && tiles * c < sm_count() && num_kb / (2 * c) >= 2 && (t_streamed || at_once(2 * c))) c *= 2;
   if (g_opt[OI_OPT_FORCE_SLICES] > 0) c = g_opt[OI_OPT_FORCE_SLICES];
   while (c > 1 && (c - 1) * ((num_kb + c - 1) / c) >= num_kb) c /= 2;   // no slice may be left without a k block
   return c;
