@@ -77,6 +77,7 @@ typedef __nv_bfloat16 bf16;
 int oi_pdl_enabled();
 void oi_fence_next_launch();   // the next kernel launched through oi_launch gets plain stream order (once)
 int oi_take_launch_fence();
+int oi_sm_count();         // multiprocessors of the device that was current at the first question (148 on a B200)
 void oi_count_launch();   // every kernel launched through oi_launch is counted (oi_launches)
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }

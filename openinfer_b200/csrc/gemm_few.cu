@@ -39,7 +39,6 @@ constexpr int kChunkK = kChunkBlocks * kWarps * 64;   // 1,024 k of a row in a s
 constexpr int kRowBytes = kChunkK * 2 + 16;
 constexpr int kPartBytes = 8192;
 constexpr int kRingBytes = 12 * 8 * kRowBytes;  // at most 194 KB
-constexpr int kSms = 148;
 
 __device__ int g_few_error = 0;                 // set when a bounded wait ran out
 
@@ -239,7 +238,7 @@ int launch(const FewArgs& args, cudaStream_t s) {
     configured = true;
   }
   a.groups = kGlu ? a.N / 16 : (a.N + 8 * G - 1) / (8 * G);
-  const int grid = a.groups < kSms ? a.groups : kSms;
+  const int sms = oi_sm_count(), grid = a.groups < sms ? a.groups : sms;
   const long long wanted = (long long)((a.groups + grid - 1) / grid) * ((a.K + kChunkK - 1) / kChunkK);
   a.stages = wanted < kMost ? (int)wanted : kMost;
   oi_launch(kernel, dim3(grid), dim3(kThreads), kPartBytes + a.stages * (kStageBytes + 16) + 16, s, a);
@@ -250,9 +249,12 @@ int launch(const FewArgs& args, cudaStream_t s) {
 template <int NT, int B, typename TOut>
 int pick_rows(const FewArgs& a, bool glu, cudaStream_t s) {
   if (glu) return launch<NT, 2, B, TOut, true>(a, s);
-  // eight rows of W at a time where that spreads them more evenly over the SMs, else sixteen
-  const int one = 8 * (((a.N + 7) / 8 + kSms - 1) / kSms), two = 16 * (((a.N + 15) / 16 + kSms - 1) / kSms);
-  return one < two ? launch<NT, 1, B, TOut, false>(a, s) : launch<NT, 2, B, TOut, false>(a, s);
+  // Sixteen rows of W at a time: a group costs a barrier and a store whatever it holds (8 rows of x, N 12288 K 1024: 5.8 us, 7.1 with
+  // groups of eight although these spread more evenly, 88 rows a CTA instead of 96; N 24576 K 3072 25.4 and 32.0; at 16 rows of x short
+  // rows of W would rather have three groups of eight than two of sixteen, N 3720 K 128 3.75 and 3.96). Eight where every
+  // CTA has one group: at 16 rows of x N 1024 K 512 0.60 and 0.67 of the streaming kernel's time, K 1024 0.65 and 0.76 (up to eight rows
+  // would rather have sixteen there too, 3.0 and 2.8 us, but a row's sums must not depend on how many rows there are).
+  return a.N <= 8 * oi_sm_count() ? launch<NT, 1, B, TOut, false>(a, s) : launch<NT, 2, B, TOut, false>(a, s);
 }
 
 template <int NT, typename TOut>

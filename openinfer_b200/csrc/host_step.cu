@@ -15,16 +15,6 @@ constexpr int kSkinnyMaxRows = 16;
 constexpr int kFusedMinRows = 128;    // rows from which gate/up forms the activation in the tcgen05 product's epilogue
 constexpr int kPair = 0;              // tile_n value that stands for 256 x 256 tiles of a pair of CTAs
 
-int sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      n = 148;
-  }
-  return n;
-}
-
 // operands that TMA can fetch: rows contiguous in k, 16-byte aligned bases and row strides
 bool tma_ok(const void* x, long long ldx, const void* w, long long ldw, int K) {
   return K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
@@ -35,33 +25,45 @@ thread_local int t_streamed = 0;
 
 // How many K slices (CTAs per cluster) the streaming kernel uses: one when the tiles of 128 weight rows alone
 // fill the GPU, else the fewest slices that give every SM a CTA, each slice at least two k blocks long, while all CTAs run at
-// once: two fit on an SM, but clusters of 8 only 33 at a time (264 CTAs), of 4 only 70 (280), and what is left over runs alone.
+// once: two fit on an SM, but clusters of 8 only 33 at a time (264 CTAs), of 4 only 71 (284), and what is left over runs alone.
 // Measured on B200 at M = 8 (us, inside a CUDA graph): N 6144 K 4096: 14.2 with 4 slices (16.1 with 2, 17.0
 // with 8); N 4096 K 4096: 11.1 with 8 (11.8 with 4); N 4096 K 12288: 20.9 with 8 (22.1 with 4); N 24576 and
 // N 151936: one slice (34.4 and 188). With the norm kernel before it, at M = 1: N 4224 K 4096: 8.4 with 8 slices (264 CTAs; 9.7
-// with 4), N 4352 9.8 with 4 (12.7 with 8, 272 CTAs); N 8960 K 4096: 14.4 with 4 (280 CTAs; 15.5 with 2), N 9216 15.7 with 2 (21.1
-// with 4, 288 CTAs). Clusters of 2 all fit, but more than 256 CTAs of short slices do not pay for their sums: N 16512 at 32 rows
+// with 4), N 4352 9.8 with 4 (12.7 with 8, 272 CTAs); N 9040 K 4672, 7 rows: 16.1 with 4 (284 CTAs; 18.2 with 2), N 9216 K 4096 15.7
+// with 2 (21.1 with 4, 288 CTAs). Clusters of 2 all fit, but more than 256 CTAs of short slices do not pay for their sums: N 16512 at 32 rows
 // K 2048 16.9 with one slice (17.8 with 2), K 3072 22.7 with 2 (23.6 with one), K 8192 49.9 (54.3).
 int stream_slices(int N, int K) {
   const int tiles = (N + 127) / 128, num_kb = (K + 63) / 64;
   auto at_once = [&](int slices) {
     const int ctas = tiles * slices;
-    return slices == 8 ? ctas <= 264 : (slices == 4 ? ctas <= 280 : ctas <= 256 || num_kb >= 48);
+    return slices == 8 ? ctas <= 264 : (slices == 4 ? ctas <= 284 : ctas <= 256 || num_kb >= 48);
   };
   int c = 1;
-  while (c < 8 && tiles * c < sm_count() && num_kb / (2 * c) >= 2 && (t_streamed || at_once(2 * c))) c *= 2;
+  while (c < 8 && tiles * c < oi_sm_count() && num_kb / (2 * c) >= 2 && (t_streamed || at_once(2 * c))) c *= 2;
   if (g_opt[OI_OPT_FORCE_SLICES] > 0) c = g_opt[OI_OPT_FORCE_SLICES];
   while (c > 1 && (c - 1) * ((num_kb + c - 1) / c) >= num_kb) c /= 2;   // no slice may be left without a k block
   return c;
 }
 
-// Whether gemm_few.cu takes a decode product: rows of up to 3,072 (figures there); longer ones, which x's rows still fit, only
-// where 148 CTAs take all of W at a time (N 2048 K 6144 6.9 us against the streaming kernel's 9.1 at 8 rows): all of x has to reach
-// every SM, and beside other long streams nothing is left of it (N 4096 K 4096 11.4 against 9.6 at 16 rows; Qwen3-8B sizes at 8
-// requests 68.2 against 68.4 ms). Nor the longest streams: N 32768 K 1024 15.0 against 14.3 at 16 rows, 13.3 against 13.6 at one.
+// Whether gemm_few.cu takes a decode product (us with the norm kernel before it, gemm_few.cu against the streaming kernel):
+// * Rows of up to 3,072. Longer ones, which x's rows still fit, only where 148 CTAs take all of W at a time (N 2048 K 6144 6.9 against
+//   9.1 at 8 rows): all of x has to reach every SM, and beside other long streams nothing is left of it (N 4096 K 4096 11.4 against
+//   9.6 at 16 rows; Qwen3-8B sizes at 8 requests 68.2 against 68.4 ms).
+// * Not the longest streams: N 32768 K 1024 15.0 against 14.3 at 16 rows, 13.3 against 13.6 at one.
+// * A CTA spends some 0.65 us on a group of 16 rows however short they are, and as long on the last stage of a row as on a
+//   full one. So the k that stages are too long for, over all groups of a CTA, are limited: K 64, 8 rows: N 6144 (2,880 of them)
+//   3.4 against 3.5, N 12288 5.4 against 3.4, N 24576 9.4 against 3.5; K 512: N 12288 (3,072) 0.94 of the time, N 20480 1.22; K 1536:
+//   N 12288 (3,072) 0.92, N 20480 1.09; K 2560: 0.95 and 1.05. K 1024 N 24576 (none) 0.88.
+// * From nine rows on, x is twice as long: K 3072 N 2048 (128 CTAs) 0.80, N 2368 and 2560 1.05 to 1.09, N 3072 1.00, N 9728 0.87;
+//   K 64 N 3072 0.96, N 5120 1.25.
 bool few_takes(const void* x, long long ldx, const void* W, long long ldw, int M, int N, int K) {
-  return !t_streamed && g_opt[OI_OPT_FORCE_SLICES] == 0 && K >= 64 && K % 64 == 0 && K <= oi_gemm_few_max_k(M) &&
-         N <= (K <= 3072 ? 24576 : 16 * 148) && ldx % 16 == 0 && ldw % 8 == 0 && (uintptr_t)x % 32 == 0 && (uintptr_t)W % 16 == 0;
+  if (t_streamed || g_opt[OI_OPT_FORCE_SLICES] != 0 || K < 64 || K % 64 || K > oi_gemm_few_max_k(M) || ldx % 16 || ldw % 8 ||
+      (uintptr_t)x % 32 || (uintptr_t)W % 16)
+    return false;
+  const int groups = ((N + 15) / 16 + oi_sm_count() - 1) / oi_sm_count();      // of 16 rows, one CTA's
+  const int spare = (1024 - K % 1024) % 1024 * groups;
+  if (M > 8 && ((K > 2048 && N > 2048 && N < 3072) || (K < 256 && groups > 2))) return false;
+  return K <= 3072 ? N <= 24576 && spare <= 3072 : groups == 1 && (M <= 8 || N <= 2048);
 }
 
 // K slices of the mma.sync decode product, 0 if it does not take the shape (a slice's activations must fit in

@@ -42,6 +42,16 @@ static unsigned long long g_launches = 0;
 void oi_count_launch() { ++g_launches; }
 OI_API unsigned long long oi_launches() { return g_launches; }
 
+int oi_sm_count() {
+  static int n = 0;
+  if (!n) {
+    int dev = 0, found = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&found, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) found = 148;
+    n = found;
+  }
+  return n;
+}
+
 OI_API int oi_set_pdl(int enabled) {
   g_pdl = enabled ? 1 : 0;
   return OI_OK;

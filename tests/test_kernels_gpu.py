@@ -1904,10 +1904,12 @@ def test_depth_averages_share_their_earlier_terms(rows, hidden, coef_dtype):
 
 
 @pytest.mark.parametrize("M,N,K,x_off,few", [
-    (4, 1024, 1024, 0, True), (16, 2368, 4096, 0, True), (8, 2368, 6144, 0, True), (16, 96, 64, 0, True),
+    (4, 1024, 1024, 0, True), (16, 2048, 4096, 0, True), (8, 2368, 6144, 0, True), (16, 96, 64, 0, True),
     (4, 1024, 1024, 8, False),                                        # rows of x 16 bytes off
     (4, 96, 1000, 0, False), (17, 1024, 1024, 0, False),              # K no multiple of 64; one row too many
-    (16, 1024, 6144, 0, False), (8, 2376, 4096, 0, False)])           # x's rows do not fit; longer rows than 148 CTAs take at a time
+    (16, 1024, 6144, 0, False), (8, 2376, 4096, 0, False),            # x's rows do not fit; longer rows than 148 CTAs take at a time
+    (8, 7104, 64, 0, True), (8, 7112, 64, 0, False), (16, 7104, 64, 0, False), (1, 24576, 512, 0, False), (8, 14208, 1536, 0, True),
+    (8, 14216, 1536, 0, False), (8, 24576, 1024, 0, True), (16, 2056, 2112, 0, False), (16, 3072, 2112, 0, True), (16, 2368, 4096, 0, False)])
 def test_which_kernel_takes_a_decode_product(M, N, K, x_off, few):
     """The dispatch's results are those of the kernel that the rule names, bit for bit."""
     from openinfer_b200.kernels import lib as klib
