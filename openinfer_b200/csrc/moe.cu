@@ -136,16 +136,15 @@ __device__ __forceinline__ void choose(float* z, unsigned char* taken, int row, 
 
 // A block takes kRows rows, a warp kExperts experts at a time for all of them, and then chooses for row after row. Few rows:
 // 1 x 1, so that a row's 16-byte loads are all in flight (a warp per four experts took 14.5 us for 4 rows of width 2,048 and
-// 16 experts, this 7.3 us), and the weights and corrections, which no kernel of a step writes, ahead of the wait (4 rows
-// in a decode step 8.7 us before, with the choices in local memory, 8.2 now; Luzitar's pass 17.56 -> 17.34 ms); many: 4 x 4, sixteen dot products for every eight loads (6,300 rows 39 us; one row a block took
-// 51 us, 4 x 1 69 us).
+// 16 experts, this 7.3 us), and the weights and corrections, which no kernel of a step writes, ahead of the wait (4 rows in a
+// decode step 8.7 us before, with the choices in local memory, 8.2 now; Luzitar's pass 17.56 -> 17.34 ms). Many: 4 x 4, sixteen
+// dot products for every eight loads (6,300 rows 39 us; one row a block took 51 us, 4 x 1 69 us).
 // kHold: 1 x 1 with no more experts than the block has warps and no more of a row than a lane holds.
 constexpr int kHoldPieces = 8, kHoldExperts = 24, kCorrCopy = 512;
 template <typename T, int kRows, int kExperts, bool kHold>
-__global__ void __launch_bounds__(kHold ? 32 * kHoldExperts : (kRows > 1 ? 512 : 1024)) moe_router_kernel(const T* x, long long ldx, const void* __restrict__ w, int w_dtype,
-                                                          int rows, int K, int E, int top, int* __restrict__ ids, float* __restrict__ wts,
-                                                          int scoring, const float* __restrict__ correction, int n_groups, int keep_groups,
-                                                          float weight_scale) {
+__global__ void __launch_bounds__(kHold ? 32 * kHoldExperts : (kRows > 1 ? 512 : 1024))
+moe_router_kernel(const T* x, long long ldx, const void* __restrict__ w, int w_dtype, int rows, int K, int E, int top, int* __restrict__ ids,
+                  float* __restrict__ wts, int scoring, const float* __restrict__ correction, int n_groups, int keep_groups, float weight_scale) {
   pdl_trigger();
   // the corrections [E] (up to kCorrCopy); per row: logits [E], scores [E], group scores [E]; then, per row, which experts are taken [E bytes]
   extern __shared__ float router_smem[];
