@@ -178,6 +178,14 @@ def current_stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+def current_device() -> int:
+    """The index of the calling thread's current device."""
+    if _raw_device is not None:
+        return _raw_device()
+    import torch
+    return torch.cuda.current_device()
+
+
 def check(code: int, what: str) -> None:
     if code != 0:
         msg = load().oi_last_error().decode(errors="replace")

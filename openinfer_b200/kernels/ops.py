@@ -5,6 +5,7 @@ the current stream. None of them has another implementation to fall back to.
 """
 from __future__ import annotations
 
+from contextlib import nullcontext
 from typing import NamedTuple, Optional
 
 import torch
@@ -107,7 +108,8 @@ class SlotClearer:
     def clear(self, slot: int) -> None:
         if not 0 <= slot < self.slots:
             raise KernelError(f"clear_slots: slot {slot} of {self.slots}")
-        with torch.cuda.device(self.table.device):       # whatever device is the calling thread's own, as a fill of the tensors would
+        # on the tensors' own device, whatever the calling thread's current one is, as a fill of them would be
+        with nullcontext() if _lib.current_device() == self.table.device.index else torch.cuda.device(self.table.device):
             _lib.check(_lib.load().oi_clear_slots(self.table.data_ptr(), len(self.tensors), self.max_bytes, slot, _stream()), "clear_slots")
 
 

@@ -59,6 +59,7 @@ def test_slots_are_cleared_on_the_tensors_own_device(monkeypatch):
     monkeypatch.setattr(torch.cuda, "device", Device)
     monkeypatch.setattr(ops, "_cuda", lambda *tensors: None)
     monkeypatch.setattr(ops, "_stream", lambda: f"stream of {current[0]}")
+    monkeypatch.setattr(ops._lib, "current_device", lambda: 1)
     monkeypatch.setattr(ops._lib, "load", lambda: Library)
     ops.SlotClearer([torch.ones(4, 3), torch.ones(4, 2, 8)]).clear(2)
     assert launched == [(torch.device("cpu"), "stream of cpu", 2, 2, 64)]
