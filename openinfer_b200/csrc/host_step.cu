@@ -54,16 +54,17 @@ int stream_slices(int N, int K) {
 //   full one. So the k that stages are too long for, over all groups of a CTA, are limited: K 64, 8 rows: N 6144 (2,880 of them)
 //   3.4 against 3.5, N 12288 5.4 against 3.4, N 24576 9.4 against 3.5; K 512: N 12288 (3,072) 0.94 of the time, N 20480 1.22; K 1536:
 //   N 12288 (3,072) 0.92, N 20480 1.09; K 2560: 0.95 and 1.05. K 1024 N 24576 (none) 0.88.
-// * From nine rows on, x is twice as long: K 3072 N 2048 (128 CTAs) 0.80, N 2368 and 2560 1.05 to 1.09, N 3072 1.00, N 9728 0.87;
-//   K 64 N 3072 0.96, N 5120 1.25.
-bool few_takes(const void* x, long long ldx, const void* W, long long ldw, int M, int N, int K) {
+// * From nine rows on, x is twice as long. K 2,304 to 3,072: N 2288 (143 CTAs) 0.80 to 0.91 of the streaming kernel's time, N 2368 to
+//   2880 1.03 to 1.13, N 3008 1.00, N 9728 0.87; K 2,112 0.93 at most. K 64 and 128: N 4736 1.0, N 5632 1.09 to 1.32, but gated (where the
+//   streaming kernel has more to do behind its products) 0.70 to 0.87.
+bool few_takes(const void* x, long long ldx, const void* W, long long ldw, int M, int N, int K, int glu) {
   if (t_streamed || g_opt[OI_OPT_FORCE_SLICES] != 0 || K < 64 || K % 64 || K > oi_gemm_few_max_k(M) || ldx % 16 || ldw % 8 ||
       (uintptr_t)x % 32 || (uintptr_t)W % 16)
     return false;
   const int groups = ((N + 15) / 16 + oi_sm_count() - 1) / oi_sm_count();      // of 16 rows, one CTA's
   const int spare = (1024 - K % 1024) % 1024 * groups;
-  if (M > 8 && ((K > 2048 && N > 2048 && N < 3072) || (K < 256 && groups > 2))) return false;
-  return K <= 3072 ? N <= 24576 && spare <= 3072 : groups == 1 && (M <= 8 || N <= 2048);
+  if (M > 8 && ((K > 2112 && N > 2288 && N < 3008) || (K < 256 && groups > 2 && !glu))) return false;
+  return K <= 3072 ? N <= 24576 && spare <= 3072 : groups == 1 && (M <= 8 || N <= 2288);
 }
 
 // K slices of the mma.sync decode product, 0 if it does not take the shape (a slice's activations must fit in
@@ -137,7 +138,7 @@ OI_API int oi_streamed_products(int on) {
 
 OI_API int oi_decode_product(void* out, int out_dtype, long long ldc, const void* x, long long ldx, const void* W, long long ldw,
                              int M, int N, int K, int glu, int act, float p0, float p1, void* stream) {
-  if (few_takes(x, ldx, W, ldw, M, N, K)) return oi_gemm_few(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, glu, act, p0, p1, stream);
+  if (few_takes(x, ldx, W, ldw, M, N, K, glu)) return oi_gemm_few(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, glu, act, p0, p1, stream);
   const int c = stream_slices(N, K);
   if (glu) return oi_gemm_stream_glu(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, c, act, p0, stream);
   if (act != OI_ACT_NONE) return oi_gemm_stream_unary(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, c, act, p0, p1, stream);

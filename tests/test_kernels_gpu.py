@@ -1904,30 +1904,56 @@ def test_depth_averages_share_their_earlier_terms(rows, hidden, coef_dtype):
 
 
 @pytest.mark.parametrize("M,N,K,x_off,few", [
-    (4, 1024, 1024, 0, True), (16, 2048, 4096, 0, True), (8, 2368, 6144, 0, True), (16, 96, 64, 0, True),
+    (4, 1024, 1024, 0, True), (16, 2288, 4096, 0, True), (8, 2368, 6144, 0, True), (16, 96, 64, 0, True),
     (4, 1024, 1024, 8, False),                                        # rows of x 16 bytes off
     (4, 96, 1000, 0, False), (17, 1024, 1024, 0, False),              # K no multiple of 64; one row too many
     (16, 1024, 6144, 0, False), (8, 2376, 4096, 0, False),            # x's rows do not fit; longer rows than 148 CTAs take at a time
-    (8, 7104, 64, 0, True), (8, 7112, 64, 0, False), (16, 7104, 64, 0, False), (1, 24576, 512, 0, False), (8, 14208, 1536, 0, True),
-    (8, 14216, 1536, 0, False), (8, 24576, 1024, 0, True), (16, 2056, 2112, 0, False), (16, 3072, 2112, 0, True), (16, 2368, 4096, 0, False)])
+    (8, 7104, 64, 0, True), (8, 7112, 64, 0, False), (1, 24576, 512, 0, False), (8, 14208, 1536, 0, True),       # stages too long for
+    (8, 14216, 1536, 0, False), (8, 24576, 1024, 0, True), (8, 24584, 1024, 0, False),                           # the rows
+    (16, 2368, 2112, 0, True), (16, 2288, 2176, 0, True), (16, 2296, 2176, 0, False), (16, 3000, 2176, 0, False),   # nine rows and more
+    (16, 3008, 2176, 0, True), (16, 2296, 4096, 0, False), (16, 4736, 192, 0, True), (16, 4744, 192, 0, False), (16, 6912, 256, 0, True)])
 def test_which_kernel_takes_a_decode_product(M, N, K, x_off, few):
-    """The dispatch's results are those of the kernel that the rule names, bit for bit."""
+    """The dispatch's results are those of the kernel that the rule names, bit for bit; gated too, where the rows divide."""
     from openinfer_b200.kernels import lib as klib
     from openinfer_b200.kernels import linear as lin
     L = klib.load()
     g = torch.Generator(device=DEV).manual_seed(M + N + K)
     x = torch.randn(M * K + 8, device=DEV, generator=g).to(torch.bfloat16)[x_off: x_off + M * K].view(M, K)
     w = (torch.randn(N, K, device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)
-    want = torch.empty(M, N, device=DEV)
-    args = (want.data_ptr(), 0, N, x.data_ptr(), K, w.data_ptr(), K, M, N, K)
     stream = torch.cuda.current_stream().cuda_stream
-    if few:
-        klib.check(L.oi_gemm_few(*args, 0, 0, 0.0, 0.0, stream), "gemm_few")
-    else:
-        klib.check(L.oi_gemm_stream(*args, L.oi_stream_slices(N, K), 0, stream), "gemm_stream")
-    got = lin.linear(x, w, out_dtype=torch.float32)
-    torch.cuda.synchronize()
-    assert torch.equal(got, want) and lin.stream_status() == 0
+    for glu in (0, 1) if N % 128 == 0 else (0,):
+        want, got = (torch.empty(M, N // 2 if glu else N, device=DEV) for _ in range(2))
+        operands = (x.data_ptr(), K, w.data_ptr(), K, M, N, K)
+        if few:
+            klib.check(L.oi_gemm_few(want.data_ptr(), 0, want.stride(0), *operands, glu, glu, 0.0, 0.0, stream), "gemm_few")
+        else:
+            klib.check(L.oi_gemm_stream(want.data_ptr(), 0, want.stride(0), *operands, L.oi_stream_slices(N, K), glu, stream), "gemm_stream")
+        if glu:
+            klib.check(L.oi_decode_product(got.data_ptr(), 0, got.stride(0), *operands, 1, 1, 0.0, 0.0, stream), "decode_product")
+        else:
+            got = lin.linear(x, w, out_dtype=torch.float32)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and lin.stream_status() == 0
+
+
+def test_gated_products_of_short_rows_stay_with_the_kernel_of_few_rows():
+    """9 to 16 rows of fewer than 256 numbers: from three groups of weight rows a CTA on the plain product goes to the streaming
+    kernel, the gated one does not."""
+    from openinfer_b200.kernels import lib as klib
+    L = klib.load()
+    M, N, K = 16, 6912, 128
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x = torch.randn(M, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)
+    stream = torch.cuda.current_stream().cuda_stream
+    for glu in (0, 1):
+        few, streamed, got = (torch.empty(M, N // 2 if glu else N, device=DEV) for _ in range(3))
+        operands = (x.data_ptr(), K, w.data_ptr(), K, M, N, K)
+        klib.check(L.oi_gemm_few(few.data_ptr(), 0, few.stride(0), *operands, glu, glu, 0.0, 0.0, stream), "gemm_few")
+        klib.check(L.oi_gemm_stream(streamed.data_ptr(), 0, streamed.stride(0), *operands, L.oi_stream_slices(N, K), glu, stream), "gemm_stream")
+        klib.check(L.oi_decode_product(got.data_ptr(), 0, got.stride(0), *operands, glu, glu, 0.0, 0.0, stream), "decode_product")
+        assert not torch.equal(few, streamed)
+        assert torch.equal(got, few if glu else streamed)
 
 
 def test_steps_with_score_routers_keep_the_streaming_product():
