@@ -25,18 +25,22 @@ thread_local int t_streamed = 0;
 
 // How many K slices (CTAs per cluster) the streaming kernel uses: one when the tiles of 128 weight rows alone
 // fill the GPU, else the fewest slices that give every SM a CTA, each slice at least two k blocks long, while all CTAs run at
-// once: two fit on an SM, but clusters of 8 only 33 at a time (264 CTAs), of 4 only 71 (284), and what is left over runs alone.
+// once: two fit on an SM, but clusters of 8 only 33 at a time (264 CTAs), of 4 some 70 (280; with 284 it depends on the kernel
+// before), and what is left over runs alone.
 // Measured on B200 at M = 8 (us, inside a CUDA graph): N 6144 K 4096: 14.2 with 4 slices (16.1 with 2, 17.0
 // with 8); N 4096 K 4096: 11.1 with 8 (11.8 with 4); N 4096 K 12288: 20.9 with 8 (22.1 with 4); N 24576 and
-// N 151936: one slice (34.4 and 188). With the norm kernel before it, at M = 1: N 4224 K 4096: 8.4 with 8 slices (264 CTAs; 9.7
-// with 4), N 4352 9.8 with 4 (12.7 with 8, 272 CTAs); N 9040 K 4672, 7 rows: 16.1 with 4 (284 CTAs; 18.2 with 2), N 9216 K 4096 15.7
-// with 2 (21.1 with 4, 288 CTAs). Clusters of 2 all fit, but more than 256 CTAs of short slices do not pay for their sums: N 16512 at 32 rows
-// K 2048 16.9 with one slice (17.8 with 2), K 3072 22.7 with 2 (23.6 with one), K 8192 49.9 (54.3).
-int stream_slices(int N, int K) {
+// N 151936: one slice (34.4 and 188). With the norm kernel before it, time by time at 1 / 16 / 32 rows: 264 CTAs, N 4224 with 8
+// slices against 4, K 2048 1.03 / 1.08 / 1.25, K 3072 0.96 / 1.00 / 0.84; 272 CTAs, N 4352 K 4096 1.29 at one row. 280 CTAs, N 8960
+// with 4 slices against 2, K 1024 0.96 / 1.03 / 0.88, K 4096 0.93 / 0.89 / 0.82; 284 CTAs, N 9088 K 1024 0.97 / 1.32 / 0.93; 288 CTAs,
+// N 9216 K 4096 1.36 / 1.30 / 1.23. Clusters of 2 all fit, but more than 256 CTAs of short slices do not pay for their sums: N 16512 with 2
+// slices against one, K 2048 0.97 / 1.04 / 1.05, K 3072 0.91 / 0.98 / 0.96, K 8192 0.89 / 0.93 / 0.92; gated, where one tile's CTA
+// would do all of the work behind them, they do: K 512 0.96 / 0.87 / 0.84.
+int stream_slices(int N, int K, int glu) {
   const int tiles = (N + 127) / 128, num_kb = (K + 63) / 64;
   auto at_once = [&](int slices) {
     const int ctas = tiles * slices;
-    return slices == 8 ? ctas <= 264 : (slices == 4 ? ctas <= 284 : ctas <= 256 || num_kb >= 48);
+    if (ctas <= 256) return true;
+    return slices == 4 ? ctas <= 280 : (slices == 2 && glu) || (num_kb >= 48 && (slices == 2 || ctas <= 264));
   };
   int c = 1;
   while (c < 8 && tiles * c < oi_sm_count() && num_kb / (2 * c) >= 2 && (t_streamed || at_once(2 * c))) c *= 2;
@@ -128,7 +132,7 @@ OI_API int oi_configure(int option, int value) {
 
 OI_API int oi_option(int option) { return option >= 0 && option < OI_OPT_COUNT ? g_opt[option] : -1; }
 
-OI_API int oi_stream_slices(int N, int K) { return stream_slices(N, K); }
+OI_API int oi_stream_slices(int N, int K) { return stream_slices(N, K, 0); }
 
 OI_API int oi_streamed_products(int on) {
   const int was = t_streamed;
@@ -139,7 +143,7 @@ OI_API int oi_streamed_products(int on) {
 OI_API int oi_decode_product(void* out, int out_dtype, long long ldc, const void* x, long long ldx, const void* W, long long ldw,
                              int M, int N, int K, int glu, int act, float p0, float p1, void* stream) {
   if (few_takes(x, ldx, W, ldw, M, N, K, glu)) return oi_gemm_few(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, glu, act, p0, p1, stream);
-  const int c = stream_slices(N, K);
+  const int c = stream_slices(N, K, glu);
   if (glu) return oi_gemm_stream_glu(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, c, act, p0, stream);
   if (act != OI_ACT_NONE) return oi_gemm_stream_unary(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, c, act, p0, p1, stream);
   return oi_gemm_stream(out, out_dtype, ldc, x, ldx, W, ldw, M, N, K, c, OI_ACT_NONE, stream);
@@ -306,13 +310,13 @@ int forward_fused_norm(const OiModelDesc* m, const OiStepDesc* st, void* stream)
     if (i == 0) {
       OI_TRY(oi_rmsnorm(st->x, st->h, nullptr, OI_BF16, L.input_norm_w, L.input_norm_dtype, nullptr, T, H, L.input_eps,
                         L.input_offset, stream));
-      OI_TRY(oi_gemm_stream(st->qkv, OI_BF16, L.qkv_rows, st->x, H, L.w_qkv, H, T, L.qkv_rows, H, stream_slices(L.qkv_rows, H),
+      OI_TRY(oi_gemm_stream(st->qkv, OI_BF16, L.qkv_rows, st->x, H, L.w_qkv, H, T, L.qkv_rows, H, stream_slices(L.qkv_rows, H, 0),
                             OI_ACT_NONE, stream));
     } else {
       OiStreamEpilogue ep = {};
       ep.ssq_in = st->ssq, ep.ssq_units = units, ep.ssq_stride = st->ssq_stride, ep.inv_width = inv_width, ep.eps = L.input_eps;
       OI_TRY(oi_gemm_stream_fused(st->qkv, OI_BF16, L.qkv_rows, xs, H, L.w_qkv, H, T, L.qkv_rows, H,
-                                  stream_slices(L.qkv_rows, H), OI_ACT_NONE, &ep, stream));
+                                  stream_slices(L.qkv_rows, H, 0), OI_ACT_NONE, &ep, stream));
     }
     // ---- attention
     OiAttnLayer a = L.attn;
@@ -320,7 +324,7 @@ int forward_fused_norm(const OiModelDesc* m, const OiStepDesc* st, void* stream)
     OI_TRY(oi_attention_layer(&st->attn_steps[L.attn_step], &a, stream));
     // ---- O + residual, and what the post norm needs
     {
-      const int c = stream_slices(H, q_dim);
+      const int c = stream_slices(H, q_dim, 0);
       OiStreamEpilogue ep = {};
       ep.residual = h, ep.ld_residual = H, ep.norm_w = L.post_norm_w, ep.norm_w_bf16 = L.post_norm_dtype == OI_BF16;
       ep.w_offset = L.post_offset, ep.xs = xs, ep.ld_xs = H, ep.ssq_out = st->ssq, ep.ssq_stride = st->ssq_stride;
@@ -332,11 +336,11 @@ int forward_fused_norm(const OiModelDesc* m, const OiStepDesc* st, void* stream)
       OiStreamEpilogue ep = {};
       ep.ssq_in = st->ssq, ep.ssq_units = units, ep.ssq_stride = st->ssq_stride, ep.inv_width = inv_width, ep.eps = L.post_eps;
       OI_TRY(oi_gemm_stream_fused(st->act, OI_BF16, L.inter, xs, H, L.w_gate_up, H, T, 2 * L.inter, H,
-                                  stream_slices(2 * L.inter, H), L.act, &ep, stream));
+                                  stream_slices(2 * L.inter, H, 1), L.act, &ep, stream));
     }
     // ---- down + residual, and what the next layer's input norm needs (the last layer: only the residual)
     {
-      const int c = stream_slices(H, L.inter);
+      const int c = stream_slices(H, L.inter, 0);
       OiStreamEpilogue ep = {};
       ep.residual = h, ep.ld_residual = H;
       if (i + 1 < m->num_layers) {

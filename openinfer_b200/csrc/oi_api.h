@@ -387,7 +387,7 @@ OI_API int oi_decode_product(void* out, int out_dtype, long long ldc, const void
 // step whose experts are chosen by scores: the last bits of the products ahead of a router decide its near ties, and
 // such a model keeps the choices it has always made). Returns what it was.
 OI_API int oi_streamed_products(int on);
-// How many K slices the streaming product uses for a shape (what oi_linear passes to oi_gemm_stream).
+// How many K slices the streaming product uses for a plain product of this shape (what oi_linear passes to oi_gemm_stream).
 OI_API int oi_stream_slices(int N, int K);
 
 // down( act(gate x) * (up x) ): out[M, hidden]. w_gate_up [2 inter, hidden] with rows in blocks of `act_block`

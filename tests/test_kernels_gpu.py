@@ -1956,6 +1956,28 @@ def test_gated_products_of_short_rows_stay_with_the_kernel_of_few_rows():
         assert torch.equal(got, few if glu else streamed)
 
 
+@pytest.mark.parametrize("N,K,glu,slices", [(16512, 512, 0, 1), (16512, 512, 1, 2), (16512, 3072, 0, 2), (8960, 640, 1, 4), (9088, 640, 1, 2)])
+def test_slices_of_a_decode_product(N, K, glu, slices):
+    """17 rows go to the streaming kernel, with the slices that the rule names: bit for bit."""
+    from openinfer_b200.kernels import lib as klib
+    L = klib.load()
+    M = 17
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    x = torch.randn(M, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)
+    stream = torch.cuda.current_stream().cuda_stream
+    operands = (x.data_ptr(), K, w.data_ptr(), K, M, N, K)
+    got = torch.empty(M, N // 2 if glu else N, device=DEV)
+    klib.check(L.oi_decode_product(got.data_ptr(), 0, got.stride(0), *operands, glu, glu, 0.0, 0.0, stream), "decode_product")
+    same = []
+    for c in (1, 2, 4):
+        out = torch.empty_like(got)
+        klib.check(L.oi_gemm_stream(out.data_ptr(), 0, out.stride(0), *operands, c, glu, stream), "gemm_stream")
+        torch.cuda.synchronize()
+        same.append(torch.equal(out, got))
+    assert same == [c == slices for c in (1, 2, 4)]
+
+
 def test_steps_with_score_routers_keep_the_streaming_product():
     """Inside ``policy.streamed_products`` this thread's products (another thread's are not meant) are the streaming kernel's bit for
     bit, and outside the few-rows kernel's."""

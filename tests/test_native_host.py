@@ -135,8 +135,8 @@ def test_steps_whose_experts_are_chosen_by_scores_run_with_streamed_products(mon
 
 
 @pytest.mark.parametrize("N,K,slices", [
-    (4096, 4096, 8), (4224, 4096, 8), (4225, 4096, 4), (4352, 4096, 4),     # 256, 264, 272 CTAs in clusters of 8
-    (6144, 4096, 4), (9088, 1024, 4), (9089, 1024, 2), (9216, 2048, 2),     # 192, 284, 288 CTAs in clusters of 4
+    (4096, 4096, 8), (4224, 4096, 8), (4225, 4096, 4), (4224, 2048, 4),     # 256, 264, 272 CTAs in clusters of 8; short slices
+    (6144, 4096, 4), (8960, 1024, 4), (8961, 1024, 2), (9216, 2048, 2),     # 192, 280, 284, 288 CTAs in clusters of 4
     (16384, 512, 2), (16512, 2048, 1), (16512, 3072, 2), (18816, 8192, 2),  # 256 and more in clusters of 2, short and long slices
     (18945, 8192, 1), (128, 64, 1), (128, 192, 1), (128, 256, 2), (128, 320, 2)])
 def test_slices_of_the_streaming_product_run_at_once(N, K, slices):
