@@ -1,8 +1,8 @@
 """y = x W^T for the projections. Which kernel takes a product is decided in native code
 (``oi_linear``, csrc/host_step.cu) by operand types, shape and options:
 
-* bfloat16 x bfloat16, up to 16 rows and not too long: the hand-written kernel of whole weight rows per CTA on mma.sync
-  (``gemm_few.cu``), which has all or much of its weights on the chip before the kernel ahead of it has finished.
+* bfloat16 x bfloat16, up to 16 rows, not too long and not beside many short rows of weights: the hand-written kernel of
+  whole weight rows per CTA on mma.sync (``gemm_few.cu``), which has all or much of its weights on the chip before the kernel ahead of it has finished.
 * bfloat16 x bfloat16 otherwise, up to 32 rows (decode): the hand-written weight-streaming kernel on the
   5th-generation tensor cores (``gemm_stream.cu``: TMA -> shared memory -> tcgen05.mma with the
   weight rows on the M side), which reads nothing but weights before the kernel ahead of it on
